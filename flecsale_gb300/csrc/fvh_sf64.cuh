@@ -19,14 +19,13 @@
 // instruction, so every input gives the IEEE result.
 //
 //   mul: the 106-bit product of the 53-bit significands from four 32x32-bit
-//        integer multiplies.
+//        integer multiplies; the rounding increment is the carry of one add.
 //   add: the smaller operand aligned with 8 extra low bits and a jammed sticky
 //        bit, integer add or subtract, renormalisation.
-//   div: long division in base 2^22 (Knuth, TAOCP vol. 2, 4.3.1): each
-//        quotient digit estimated from an FP32 reciprocal of the divisor's top
-//        24 bits, then corrected by one step either way from the exact integer
-//        remainder; 53 quotient bits plus a guard bit, the final remainder
-//        gives the sticky bit.
+//   div: long division (Knuth, TAOCP vol. 2, 4.3.1) in digits of 18, 18 and 17
+//        bits, each estimated from below from an FP32 reciprocal of the
+//        divisor's top 24 bits; the exact integer remainder stays in
+//        [0, 1.5 divisors) and is corrected once, after the last digit.
 //
 // The tests of the exponent and zero bits work on the two 32-bit halves taken
 // through an opaque move, so the compiler cannot turn them into FP64
@@ -80,31 +79,61 @@ __device__ __forceinline__ bool is_finite(unsigned hi) {
   return (hi & 0x7ff00000u) != 0x7ff00000u;
 }
 
-// Rounded product of two moderate operands (halves al:ah, bl:bh); sign and
-// exponent are left to the caller through `sign`.
-__device__ __forceinline__ double mul_core(unsigned al, unsigned ah, unsigned bl, unsigned bh,
-                                           unsigned ea, unsigned eb, unsigned sign) {
-  // significands (53 bits): (mah:al), (mbh:bl); P = product in 32-bit words
-  // w3 w2 w1 w0, P in [2^104, 2^106)
-  const unsigned mah = (ah & 0xfffffu) | 0x100000u, mbh = (bh & 0xfffffu) | 0x100000u;
-  const unsigned long long p0 = (unsigned long long)al * bl;
+// An operand taken apart: the significand (m : lo), 53 bits with the implied
+// one, and the sign and exponent field as they stand in the high half.
+struct parts {
+  unsigned lo, m, se;
+  bool zero;
+};
+
+// Takes x apart; `rare` collects whether it is neither moderate nor a zero.
+__device__ __forceinline__ parts take(double x, unsigned &rare) {
+  unsigned lo, hi;
+  halves(x, lo, hi);
+  parts p;
+  p.lo = lo;
+  p.m = (hi & 0xfffffu) | 0x100000u;
+  p.se = hi & 0xfff00000u;
+  const unsigned h = hi & 0x7fffffffu;
+  p.zero = (h | lo) == 0u;
+  rare |= (unsigned)!((h - (523u << 20) < (1001u << 20)) | p.zero);
+  return p;
+}
+
+// Rounded product of two moderate operands.  The sign and exponent fields are
+// added as they stand: modulo 2^32 the sign bits add to their exclusive or.
+__device__ __forceinline__ double mul_core(const parts &a, const parts &b) {
+  // P = product of the significands in 32-bit words w3 w2 w1 w0, in [2^104, 2^106)
+  const unsigned long long p0 = (unsigned long long)a.lo * b.lo;
   const unsigned long long t =
-      (unsigned long long)al * mbh + (unsigned long long)mah * bl + (p0 >> 32);
-  const unsigned long long u = (unsigned long long)mah * mbh + (t >> 32);
+      (unsigned long long)a.m * b.lo + ((unsigned long long)a.lo * b.m + (p0 >> 32));
+  const unsigned long long u = (unsigned long long)a.m * b.m + (t >> 32);
   const unsigned w0 = (unsigned)p0, w1 = (unsigned)t, w2 = (unsigned)u, w3 = (unsigned)(u >> 32);
-  // the significand is P >> (32 + s), s = 20, or 21 when P >= 2^105
-  const unsigned top = (w3 >> 9) & 1u;
-  const unsigned s = 20u + top;
-  const unsigned mlo = __funnelshift_r(w1, w2, s), mhi = __funnelshift_r(w2, w3, s);
-  const unsigned guard = (w1 >> (s - 1u)) & 1u;
-  const unsigned sticky = ((w1 << (33u - s)) | w0) != 0u;
-  const unsigned inc = guard & (sticky | (mlo & 1u));
+  // shifted left by s the significand of the result is the words above w1
+  const unsigned top = w3 >> 9, s = 12u - top;  // top = 1 when P >= 2^105
+  const unsigned mhi = __funnelshift_l(w2, w3, s), mlo = __funnelshift_l(w1, w2, s);
+  // what is below it, w0 jammed into the lowest bit (bit s after the shift),
+  // and the result's lowest bit in bit 0: above 2^31 it rounds up, so adding
+  // 2^31 - 1 carries exactly then
+  const unsigned f = ((w1 | (w0 < 1u ? w0 : 1u)) << s) | (mlo & 1u);
   // exponent field of the result minus one (the significand's leading one,
   // bit 52, adds it back; a rounding carry to 2^53 moves on to the exponent)
-  const unsigned e1 = ea + eb - 1024u + top;
-  const unsigned long long r =
-      ((unsigned long long)(mhi + (e1 << 20)) << 32 | mlo) + (unsigned long long)inc;
-  return dbl(r | ((unsigned long long)sign << 32));
+  const unsigned e1 = a.se + b.se - (1024u << 20) + (top << 20);
+  unsigned lo, hi;
+  asm("{\n\t.reg .u32 t;\n\t"
+      "add.cc.u32 t, %2, 0x7fffffff;\n\t"
+      "addc.cc.u32 %0, %3, 0;\n\t"
+      "addc.u32 %1, %4, %5;\n\t}"
+      : "=r"(lo), "=r"(hi)
+      : "r"(f), "r"(mlo), "r"(mhi), "r"(e1));
+  return join(lo, hi);
+}
+
+// Product of two operands taken apart, zeros by a select (the sign of a
+// product is that of the added sign bits).
+__device__ __forceinline__ double mul_parts(const parts &a, const parts &b) {
+  const double q = mul_core(a, b);
+  return (a.zero | b.zero) ? join(0u, (a.se + b.se) & 0x80000000u) : q;
 }
 
 // a * b
@@ -120,7 +149,8 @@ __device__ __forceinline__ double mul(double a, double b) {
       return join(0u, sign);
     return mul_rare(a, b);
   }
-  return mul_core(al, ah, bl, bh, ea, eb, sign);
+  unsigned rare = 0;
+  return mul_core(take(a, rare), take(b, rare));
 }
 
 // a + b
@@ -178,64 +208,50 @@ __device__ __forceinline__ double sub(double a, double b) {
   return add(a, join(bl, bh ^ 0x80000000u));
 }
 
-// The integer v < 2^24 as a float, without the int-to-float conversion
-// instruction: 2^23 + (v mod 2^23) by bit assembly, then 2^23 taken off again
-// when v < 2^23.
-__device__ __forceinline__ float u24_to_float(unsigned v) {
-  const float f = __int_as_float(0x4b000000 | (v & 0x7fffffu));
-  return (v >> 23) ? f : f - 8388608.0f;
-}
-
-// One quotient digit of K bits: q = floor(r 2^K / d), r <- r 2^K - q d, for
-// 0 <= r < d, 2^52 <= d < 2^53.  ginv = 2^K / float(d >> 29) (FP32 reciprocal,
-// relative error below 2^-23).  The estimate floor(float(r >> 29) * ginv) is
-// within one of q: truncating r and d and the reciprocal's error each move
-// r 2^K / d by less than 1/2 for K <= 22; the remainder, exact in 64-bit
-// two's complement, then corrects it.
+// One quotient digit of K <= 18 bits: q <= r 2^K / d, r <- r 2^K - q d, for
+// 0 <= r < 2 d, 2^52 <= d < 2^53 (nd = 2^64 - d).  ginv is 2^(K+2) times an
+// FP32 reciprocal of dh = d >> 29 lowered by 2^-21.  With fr = r >> 31 < 2^23
+// the estimate floor(fr ginv) never exceeds r 2^K / d: truncating d and the
+// reciprocal's error raise it by less than 2^-22 of itself.  It falls short by
+// less than 1.49 (1 for the floor, 2^(K-21) for truncating r, 0.36 for the
+// lowered reciprocal at a digit below 2^19), so 0 <= r < 1.49 d again.  The
+// remainder is exact modulo 2^64.
 template <int K>
-__device__ __forceinline__ unsigned div_digit(unsigned long long &r, unsigned long long d,
+__device__ __forceinline__ unsigned div_digit(unsigned long long &r, unsigned long long nd,
                                               float ginv) {
-  const float fr = u24_to_float((unsigned)(r >> 29));
+  const float fr = __int_as_float(0x4b000000 | (int)(unsigned)(r >> 31)) - 8388608.0f;
   // floor(fr * ginv) for a value below 2^23: round toward zero onto 2^23
-  const float qf = __fmaf_rz(fr, ginv, 8388608.0f);
-  unsigned q = (unsigned)__float_as_int(qf) & 0x7fffffu;
-  long long rr = (long long)((r << K) - (unsigned long long)q * d);
-  if (rr < 0) {
-    q -= 1;
-    rr += (long long)d;
-  }
-  if (rr >= (long long)d) {
-    q += 1;
-    rr -= (long long)d;
-  }
-  r = (unsigned long long)rr;
+  const unsigned q = (unsigned)__float_as_int(__fmaf_rz(fr, ginv, 8388608.0f)) & 0x7fffffu;
+  r = (r << K) + (unsigned long long)q * (unsigned)nd +
+      ((unsigned long long)(q * (unsigned)(nd >> 32)) << 32);
   return q;
 }
 
 // Rounded quotient of two moderate operands.
-__device__ __forceinline__ double div_core(unsigned al, unsigned ah, unsigned bl, unsigned bh,
-                                           unsigned ea, unsigned eb, unsigned sign) {
-  unsigned long long x = ((unsigned long long)((ah & 0xfffffu) | 0x100000u) << 32) | al;
-  const unsigned long long d = ((unsigned long long)((bh & 0xfffffu) | 0x100000u) << 32) | bl;
+__device__ __forceinline__ double div_core(const parts &a, const parts &b) {
+  unsigned long long x = ((unsigned long long)a.m << 32) | a.lo;
+  const unsigned long long d = ((unsigned long long)b.m << 32) | b.lo;
   const bool lt = x < d;
-  const unsigned e1 = ea - eb + 1022u - (unsigned)lt;  // exponent field of the quotient - 1
-  x <<= lt;  // d <= x < 2d: the quotient's leading bit is one
-  unsigned long long r = x - d;
-  const unsigned dh = (unsigned)(d >> 29);                           // in [2^23, 2^24)
-  const float fd = __int_as_float(0x4b000000 | (dh & 0x7fffffu));  // == dh
+  x = lt ? x + x : x;  // d <= x < 2d: the quotient is in [1, 2)
+  const unsigned long long nd = 0ull - d;
+  // dh = d >> 29 in [2^23, 2^24), exactly a float
+  const float fd = __int_as_float(0x4b000000 | ((unsigned)(d >> 29) & 0x7fffffu));
   float inv;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(fd));
-  // 52 quotient bits below the leading one plus the guard bit: 22 + 22 + 9
-  const unsigned q1 = div_digit<22>(r, d, inv * 4194304.0f);
-  const unsigned q2 = div_digit<22>(r, d, inv * 4194304.0f);
-  const unsigned q3 = div_digit<9>(r, d, inv * 512.0f);
-  const unsigned long long Q = (1ull << 53) | ((unsigned long long)q1 << 31) |
-                               ((unsigned long long)q2 << 9) | q3;
-  unsigned long long m = Q >> 1;
-  const unsigned guard = (unsigned)Q & 1u;
-  const unsigned sticky = r != 0;
-  m += guard & (sticky | ((unsigned)m & 1u));
-  return dbl((((unsigned long long)e1 << 52) + m) | ((unsigned long long)sign << 32));
+  const float g18 = inv * (1048576.0f * (1.0f - 0x1p-21f));
+  unsigned long long r = x;
+  const unsigned q1 = div_digit<18>(r, nd, g18);
+  const unsigned q2 = div_digit<18>(r, nd, g18);
+  const unsigned q3 = div_digit<17>(r, nd, 0.5f * g18);
+  // Q = floor(x 2^53 / d) in [2^53, 2^54): 53 bits and the guard bit.  A
+  // quotient of two 53-bit significands is never halfway between two results
+  // (d would have to be a multiple of 2^53), so the guard bit alone rounds.
+  unsigned long long Q = (((unsigned long long)q1 << 18) + q2) * 131072ull + q3;
+  Q += (unsigned long long)(r >= d) + 1ull;
+  const unsigned long long m = Q >> 1;
+  // exponent field minus one, and the sign (see mul_core)
+  const unsigned e1 = a.se - b.se + ((lt ? 1021u : 1022u) << 20);
+  return join((unsigned)m, (unsigned)(m >> 32) + e1);
 }
 
 // a / b
@@ -250,7 +266,8 @@ __device__ __forceinline__ double div(double a, double b) {
     if (is_zero(al, ah) & is_finite(bh) & !is_zero(bl, bh)) return join(0u, sign);
     return div_rare(a, b);
   }
-  return div_core(al, ah, bl, bh, ea, eb, sign);
+  unsigned rare = 0;
+  return div_core(take(a, rare), take(b, rare));
 }
 
 // ---------------------------------------------------------------------------
@@ -261,34 +278,15 @@ __device__ __forceinline__ double div(double a, double b) {
 // instructions.  A kernel then has no branch per operation.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double mul_opt(double a, double b, unsigned &rare) {
-  unsigned al, ah, bl, bh;
-  halves(a, al, ah);
-  halves(b, bl, bh);
-  // A zero times a finite value is a zero; (a zero) & finite(b) | (b zero) &
-  // finite(a) is (either zero) & finite(a) & finite(b).  Fewer instructions
-  // than testing each case apart (2D FP64 step 1.474 -> 1.451 ms).
-  const unsigned ha = ah & 0x7fffffffu, hb = bh & 0x7fffffffu;
-  const unsigned ea = ha >> 20, eb = hb >> 20;
-  const unsigned sign = (ah ^ bh) & 0x80000000u;
-  const bool zero = ((ha | al) == 0u) | ((hb | bl) == 0u);
-  const bool fast = moderate(ea) & moderate(eb);
-  rare |= (unsigned)!(fast | (zero & (ea != 0x7ffu) & (eb != 0x7ffu)));
-  const double q = mul_core(al, ah, bl, bh, ea, eb, sign);
-  return zero ? join(0u, sign) : q;
+  const parts pa = take(a, rare), pb = take(b, rare);
+  return mul_parts(pa, pb);
 }
 
 __device__ __forceinline__ double div_opt(double a, double b, unsigned &rare) {
-  unsigned al, ah, bl, bh;
-  halves(a, al, ah);
-  halves(b, bl, bh);
-  const unsigned ea = expo(ah), eb = expo(bh);
-  const unsigned sign = (ah ^ bh) & 0x80000000u;
-  const bool za = is_zero(al, ah);
-  const bool fast = moderate(ea) & moderate(eb);
-  const bool zero = za & is_finite(bh) & !is_zero(bl, bh);
-  rare |= (unsigned)!(fast | zero);
-  const double q = div_core(al, ah, bl, bh, ea, eb, sign);
-  return za ? join(0u, sign) : q;
+  const parts pa = take(a, rare), pb = take(b, rare);
+  rare |= (unsigned)pb.zero;
+  const double q = div_core(pa, pb);
+  return pa.zero ? join(0u, (pa.se + pb.se) & 0x80000000u) : q;
 }
 
 }  // namespace sf64

@@ -76,7 +76,25 @@ __device__ __noinline__ double add_call(double a, double b) { return sf64::add(a
 // Products and quotients of one unit of work: on the integer pipes, noting
 // any operand they leave to the hardware ...
 struct arith_opt {
+  using part = sf64::parts;
   unsigned rare = 0;
+  // an operand of several products is taken apart once
+  __device__ __forceinline__ part take(double x) { return sf64::take(x, rare); }
+  // an entry of the solver's tables, known to be moderate or zero
+  __device__ __forceinline__ part take_entry(double x) { return sf64::take_plain(x); }
+  __device__ __forceinline__ double prod(const part &a, const part &b) {
+    return sf64::mul_parts(a, b);
+  }
+  // s + a * b for a sum s that started at +0 (so it is never -0 and a zero
+  // product leaves it as it is); the first product is the sum 0 + a * b
+  __device__ __forceinline__ void add_first(double &s, const part &a, const part &b) {
+    const double q = sf64::mul_core(a, b);
+    s = (a.zero | b.zero) ? 0.0 : q;
+  }
+  __device__ __forceinline__ void add(double &s, const part &a, const part &b) {
+    const double q = sf64::mul_core(a, b);
+    if (!(a.zero | b.zero)) s += q;
+  }
   __device__ __forceinline__ double mul(double a, double b) {
     const flagged r = mul_call(a, b);
     rare |= r.rare;
@@ -100,6 +118,15 @@ struct arith_opt {
 };
 // ... and with the FP64 instructions (the evaluation kept when `rare`)
 struct arith_hw {
+  static constexpr unsigned rare = 0;
+  using part = double;
+  __device__ __forceinline__ part take(double x) { return x; }
+  __device__ __forceinline__ part take_entry(double x) { return x; }
+  __device__ __forceinline__ double prod(part a, part b) { return __dmul_rn(a, b); }
+  __device__ __forceinline__ void add_first(double &s, part a, part b) {
+    s = 0.0 + __dmul_rn(a, b);
+  }
+  __device__ __forceinline__ void add(double &s, part a, part b) { s += __dmul_rn(a, b); }
   __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
   __device__ __forceinline__ double quo(double a, double b) { return __ddiv_rn(a, b); }
   __device__ __forceinline__ double half(double x) { return __dmul_rn(x, 0.5); }
@@ -179,12 +206,23 @@ __device__ __forceinline__ double absval(double x) {
 __device__ __forceinline__ double smax(double a, double b) { return lt(a, b) ? b : a; }
 __device__ __forceinline__ double smin(double a, double b) { return lt(b, a) ? b : a; }
 
+// x with a negative zero made positive: 0 + x without an FP64 addition.
+__device__ __forceinline__ double plus_zero(double x) {
+  unsigned lo, hi;
+  sf64::halves(x, lo, hi);
+  return sf64::join(lo, (hi ^ 0x80000000u | lo) == 0u ? 0u : hi);
+}
+
+// The reference sums from zero in index order.  Starting from the first
+// product instead gives the same sum except that it can be -0 (all products
+// -0), where the sum from zero is +0.  The FP64 pipe is the bound of these
+// kernels, and this takes one addition off every dot product.
 template <int D, class A>
 __device__ __forceinline__ double dot(A &ar, const double *a, const double *b) {
-  double s = 0;
+  double s = ar.mul(a[0], b[0]);
 #pragma unroll
-  for (int i = 0; i < D; ++i) s += ar.mul(a[i], b[i]);
-  return s;
+  for (int i = 1; i < D; ++i) s += ar.mul(a[i], b[i]);
+  return plus_zero(s);
 }
 
 // Same slots as pack_copy(c, d, v, p, e, T, a) (tasks.h:420).  T is carried by
@@ -196,13 +234,18 @@ struct prim {
 
 template <int D, class A>
 __device__ __forceinline__ double total_energy(A &ar, const prim<D> &u) {
-  return u.e + ar.half(dot<D>(ar, u.v, u.v));  // 0.5 * |v|^2
+  // 0.5 * |v|^2; squares are never -0
+  double s = ar.mul(u.v[0], u.v[0]);
+#pragma unroll
+  for (int i = 1; i < D; ++i) s += ar.mul(u.v[i], u.v[i]);
+  return u.e + ar.half(s);
 }
 
+// The physical flux of u along n from its normal velocity vn = v.n and total
+// energy et, which the Riemann fluxes also use themselves.
 template <int D, class A>
-__device__ __forceinline__ void phys_flux(A &ar, const prim<D> &u, const double *n, double *f) {
-  const double et = total_energy<D>(ar, u);
-  const double vn = dot<D>(ar, u.v, n);
+__device__ __forceinline__ void phys_flux(A &ar, const prim<D> &u, const double *n, double vn,
+                                          double et, double *f) {
   const double mass_flux = ar.mul(u.d, vn);
   f[0] = mass_flux;
 #pragma unroll
@@ -210,11 +253,25 @@ __device__ __forceinline__ void phys_flux(A &ar, const prim<D> &u, const double 
   f[D + 1] = ar.mul(mass_flux, et + ar.quo(u.p, u.d));
 }
 
+// a or b, value by value (a reference to either would put both in memory)
+template <int D>
+__device__ __forceinline__ prim<D> pick(bool first, const prim<D> &a, const prim<D> &b) {
+  prim<D> u;
+  u.d = first ? a.d : b.d;
+#pragma unroll
+  for (int i = 0; i < D; ++i) u.v[i] = first ? a.v[i] : b.v[i];
+  u.p = first ? a.p : b.p;
+  u.e = first ? a.e : b.e;
+  u.a = first ? a.a : b.a;
+  return u;
+}
+
+// ur - ul of the conserved variables, from the total energies
 template <int D, class A>
 __device__ __forceinline__ void solution_delta(A &ar, const prim<D> &l, const prim<D> &r,
-                                               double *du) {
-  const double ener_l = ar.mul(l.d, total_energy<D>(ar, l));
-  const double ener_r = ar.mul(r.d, total_energy<D>(ar, r));
+                                               double et_l, double et_r, double *du) {
+  const double ener_l = ar.mul(l.d, et_l);
+  const double ener_r = ar.mul(r.d, et_r);
   du[0] = r.d - l.d;
 #pragma unroll
   for (int i = 0; i < D; ++i) du[1 + i] = ar.mul(r.d, r.v[i]) - ar.mul(l.d, l.v[i]);
@@ -230,14 +287,17 @@ __device__ __forceinline__ void hlle(A &ar, const prim<D> &l, const prim<D> &r,
   // one physical-flux evaluation per side: the upwind side's (or the left
   // side's when both are needed), then the right side's if both are
   const bool up_l = ge0(lambda_l), up_r = !up_l && le0(lambda_r);
-  phys_flux<D>(ar, up_r ? r : l, n, f);
+  const prim<D> u = pick<D>(up_r, r, l);
+  const double et = total_energy<D>(ar, u);
+  phys_flux<D>(ar, u, n, up_r ? vnr : vnl, et, f);
   if (up_l || up_r) return;
   double fr[D + 2], du[D + 2];
-  phys_flux<D>(ar, r, n, fr);
+  const double et_r = total_energy<D>(ar, r);
+  phys_flux<D>(ar, r, n, vnr, et_r, fr);
   const double c1 = ar.mul(lambda_l, lambda_r);
   const double c2 = lambda_r - lambda_l;
   const double c2inv = ar.quo(1, c2);
-  solution_delta<D>(ar, l, r, du);
+  solution_delta<D>(ar, l, r, et, et_r, du);
 #pragma unroll
   for (int i = 0; i < D + 2; ++i)
     f[i] = ar.mul(c2inv, ar.mul(lambda_r, f[i]) - ar.mul(lambda_l, fr[i]) + ar.mul(c1, du[i]));
@@ -247,15 +307,15 @@ template <int D, class A>
 __device__ __forceinline__ void rusanov(A &ar, const prim<D> &l, const prim<D> &r,
                                         const double *n, double *f) {
   double fl[D + 2], fr[D + 2], du[D + 2];
+  const double vnl = dot<D>(ar, l.v, n), vnr = dot<D>(ar, r.v, n);
+  const double et_l = total_energy<D>(ar, l), et_r = total_energy<D>(ar, r);
   {
     fp64_products<A> pp{ar};
-    phys_flux<D>(pp, l, n, fl);
+    phys_flux<D>(pp, l, n, vnl, et_l, fl);
   }
-  phys_flux<D>(ar, r, n, fr);
-  const double sl = l.a + absval(dot<D>(ar, l.v, n));
-  const double sr = r.a + absval(dot<D>(ar, r.v, n));
-  const double s = smax(sl, sr);
-  solution_delta<D>(ar, l, r, du);
+  phys_flux<D>(ar, r, n, vnr, et_r, fr);
+  const double s = smax(l.a + absval(vnl), r.a + absval(vnr));
+  solution_delta<D>(ar, l, r, et_l, et_r, du);
   const double half_s = ar.half(s);  // s / 2
 #pragma unroll
   for (int i = 0; i < D + 2; ++i) f[i] = ar.half(fl[i] + fr[i]) - ar.mul(du[i], half_s);
@@ -279,16 +339,17 @@ __device__ __forceinline__ void hllc(A &ar, const prim<D> &l, const prim<D> &r,
     sM = ar.quo(r.p - l.p + ar.mul(ml, vnl) - ar.mul(mr, vnr), ml - mr);
     left = ge0(sM);
   }
-  const prim<D> &u = left ? l : r;
+  const prim<D> u = pick<D>(left, l, r);
+  const double vnK = left ? vnl : vnr;
+  const double et = total_energy<D>(ar, u);
   {
     fp64_products<A> pp{ar};
-    phys_flux<D>(pp, u, n, f);
+    phys_flux<D>(pp, u, n, vnK, et, f);
   }
   if (!star) return;
   const double sK = left ? sL : sR;
   const double mK = left ? ml : mr;
-  const double vnK = left ? vnl : vnr;
-  const double EK = ar.mul(u.d, total_energy<D>(ar, u));
+  const double EK = ar.mul(u.d, et);
   const double fac = ar.quo(mK, sK - sM);
   const double dvn = sM - vnK;
   f[0] = f[0] + ar.mul(sK, fac - u.d);
@@ -450,9 +511,16 @@ __device__ __forceinline__ void lsq_matrix(A &ar, const fvh_mesh_view &m, int c0
   }
 }
 
+// notes an offset that is neither zero nor within 2^+-500 (take_entry)
+__device__ __forceinline__ void note_odd(double x, unsigned *odd) {
+  unsigned rare = 0;
+  sf64::take(x, rare);
+  if (rare) atomicOr(odd, 1u);
+}
+
 template <int D>
 __global__ void cell_tables_kernel(const fvh_mesh_view m, double *lsq, double *slot_dx,
-                                   double *nbr_dx, double *vtx_dx) {
+                                   double *nbr_dx, double *vtx_dx, unsigned *odd) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.num_cells) return;
   arith_hw hw;  // set-up, once per mesh
@@ -473,7 +541,11 @@ __global__ void cell_tables_kernel(const fvh_mesh_view m, double *lsq, double *s
   for (int q = m.cell_nbr_offsets[c]; q < m.cell_nbr_offsets[c + 1]; ++q) {
     const int c1 = m.cell_nbrs[q];
 #pragma unroll
-    for (int d = 0; d < D; ++d) nbr_dx[(size_t)q * D + d] = m.cell_centroid[d][c1] - x0[d];
+    for (int d = 0; d < D; ++d) {
+      const double dx = m.cell_centroid[d][c1] - x0[d];
+      nbr_dx[(size_t)q * D + d] = dx;
+      note_odd(dx, odd);
+    }
   }
   for (int q = m.cell_vertex_offsets[c]; q < m.cell_vertex_offsets[c + 1]; ++q) {
     const int v = m.cell_vertices[q];
@@ -483,7 +555,7 @@ __global__ void cell_tables_kernel(const fvh_mesh_view m, double *lsq, double *s
 }
 
 template <int D>
-__global__ void face_tables_kernel(const fvh_mesh_view m, double *face_dx) {
+__global__ void face_tables_kernel(const fvh_mesh_view m, double *face_dx, unsigned *odd) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= m.num_faces) return;
   const int2 cc = reinterpret_cast<const int2 *>(m.face_cells)[f];
@@ -491,9 +563,11 @@ __global__ void face_tables_kernel(const fvh_mesh_view m, double *face_dx) {
   for (int side = 0; side < 2; ++side) {
     const int c = side == 0 ? cc.x : cc.y;
 #pragma unroll
-    for (int i = 0; i < D; ++i)
-      face_dx[(size_t)f * 2 * D + side * D + i] =
-          c >= 0 ? m.face_centroid[i][f] - m.cell_centroid[i][c] : 0.0;
+    for (int i = 0; i < D; ++i) {
+      const double dx = c >= 0 ? m.face_centroid[i][f] - m.cell_centroid[i][c] : 0.0;
+      face_dx[(size_t)f * 2 * D + side * D + i] = dx;
+      note_odd(dx, odd);
+    }
   }
 }
 
@@ -531,261 +605,482 @@ __device__ __forceinline__ double *grad_plane(const fvh_gradient_view &g, int k,
                                       : k == D + 2 ? g.pressure[i] : g.sound_speed[i];
 }
 
-template <int D, int K0, int NK>
-__device__ __forceinline__ void load_values(const fvh_state_view &s, int c, double *u) {
+// ... and the limiter's view of them.  Both views hold their plane pointers one
+// after another, so a variable that is only known at run time is an index.
+template <int D>
+__device__ __forceinline__ const double *state_plane_at(const fvh_state_view &s, int k) {
+  // density, velocity[3], internal_energy, pressure, temperature, sound_speed
+  return reinterpret_cast<const double *const *>(&s)[k <= D ? k : k == D + 3 ? 7 : k + 3 - D];
+}
+template <int D>
+__device__ __forceinline__ double *const *grad_planes_at(const fvh_gradient_view &g, int k) {
+  // density[3], velocity[3][3], internal_energy[3], pressure[3], sound_speed[3]
+  return reinterpret_cast<double *const *>(&g) + 3 * (k <= D ? k : k + 3 - D);
+}
+static_assert(sizeof(fvh_state_view) == 8 * sizeof(double *) &&
+                  sizeof(fvh_gradient_view) == 21 * sizeof(double *),
+              "plane pointers stand one after another");
+
+template <int D, bool PRE>
+__device__ __forceinline__ void vertex_offset(const fvh_mesh_view &m, const tables &t, int rr,
+                                              const double *x0, double *dxv) {
+  if (PRE) {
+    load_dx<D>(t.vtx_dx + (size_t)rr * D, dxv);
+  } else {
+    const int vtx = m.cell_vertices[rr];
 #pragma unroll
-  for (int k = 0; k < NK; ++k) u[k] = state_plane<D>(s, K0 + k)[c];
+    for (int i = 0; i < D; ++i) dxv[i] = m.vertex_coord[i][vtx] - x0[i];
+  }
 }
 
-// The limited gradients gu of cell c0 for the reconstructed variables
-// K0 .. K0+NK-1 (of d, v.., e, p, a).  Each variable's gradient and limiter
-// depend on that variable alone, so the variables can be taken in groups, each
-// in its own pass over the neighbours (fewer live registers, same results).
-template <int D, int K0, int NK, bool LIMIT, bool PRE, class A>
-__device__ __forceinline__ void cell_gradients(A &ar, const fvh_mesh_view &m,
-                                               const fvh_state_view &s, const tables &t,
-                                               int c0, double (&gu)[NK][D]) {
-  constexpr int NV = NK;
-  constexpr int W = lsq_width<D>::value;
+// The limiter factor phi of one variable (tasks.h:267-299) with the reference's
+// arithmetic: u0 and the gradient g of cell c0, `plane` the variable's values.
+// Out of line: the kernel calls it only where its FP32 bounds do not decide.
+//
+// phi = min over vertices of (umax-u0)/du or (umin-u0)/du.  Correctly rounded
+// division is monotone in the divisor, so only the largest du > tol and the
+// smallest du < -tol can set the minimum; the result equals the reference's
+// per-vertex minimum.
+template <int D, bool PRE>
+__device__ __noinline__ double limiter_exact(const fvh_mesh_view &m, const tables &t,
+                                             const double *__restrict__ plane, int c0, double u0,
+                                             double g0, double g1, double g2) {
   constexpr double tol = 1.e-9;
+  const long long ktol = okey(tol), kntol = okey(-tol);
+  const double g[3] = {g0, g1, g2};
   double x0[D];
   if (!PRE) {
 #pragma unroll
     for (int i = 0; i < D; ++i) x0[i] = m.cell_centroid[i][c0];
   }
-  double u0[NV];
-  load_values<D, K0, NK>(s, c0, u0);
-  double dudx[NV][D];
+  long long kpos = 0, kneg = 0;
+  const int r0 = m.cell_vertex_offsets[c0], r1 = m.cell_vertex_offsets[c0 + 1];
+#pragma unroll 1
+  for (int rr = r0; rr < r1; ++rr) {
+    double dxv[D];
+    vertex_offset<D, PRE>(m, t, rr, x0, dxv);
+    double u1 = u0;
 #pragma unroll
-  for (int k = 0; k < NV; ++k)
+    for (int i = 0; i < D; ++i) u1 += __dmul_rn(dxv[i], g[i]);
+    const long long kd = okey(u1 - u0);
+    if (kd > ktol) kpos = (kpos < kd) ? kd : kpos;
+    else if (kd < kntol) kneg = (kd < kneg) ? kd : kneg;
+  }
+  long long kphi = okey(1.0);
+  if (kpos > ktol || kneg < kntol) {
+    // the neighbour extrema umin / umax (tasks.h:232-236)
+    long long kmin = okey(u0), kmax = kmin;
+    const int q0 = m.cell_nbr_offsets[c0], q1 = m.cell_nbr_offsets[c0 + 1];
+#pragma unroll 4
+    for (int q = q0; q < q1; ++q) {
+      const long long k1 = okey(plane[m.cell_nbrs[q]]);
+      kmin = (k1 < kmin) ? k1 : kmin;  // std::min(u1, umin)
+      kmax = (kmax < k1) ? k1 : kmax;  // std::max(u1, umax)
+    }
+    // RN(N / du) >= 1 exactly when |N| >= |du| (N and du of one sign, du
+    // normal), so the quotient is formed only when it can lower phi below 1
+    if (kpos > ktol) {
+      const double num = from_okey(kmax) - u0;
+      if (okey(num) < kpos) {
+        const long long kq = okey(__ddiv_rn(num, from_okey(kpos)));
+        kphi = (kq < kphi) ? kq : kphi;
+      }
+    }
+    if (kneg < kntol) {
+      const double num = from_okey(kmin) - u0;
+      if (okey(num) > kneg) {
+        const long long kq = okey(__ddiv_rn(num, from_okey(kneg)));
+        kphi = (kq < kphi) ? kq : kphi;
+      }
+    }
+  }
+  kphi = (kphi < 0) ? 0 : kphi;  // std::max(phi, 0)
+  return from_okey(kphi);
+}
+
+// x truncated to FP32 (relative error below 2^-23; 0 for |x| < 2^-60); `wide`
+// collects whether |x| >= 2^60 or x is a NaN.
+__device__ __forceinline__ float truncated(double x, unsigned &wide) {
+  unsigned lo, hi;
+  sf64::halves(x, lo, hi);
+  const unsigned h = hi & 0x7fffffffu;
+  wide |= (unsigned)(h >= (1083u << 20));
+  const unsigned mag = __funnelshift_l(lo, h - (896u << 20), 3);
+  return __uint_as_float(h < (963u << 20) ? 0u : mag | (hi & 0x80000000u));
+}
+
+// Order key of the high half of a double: for differences it finds the largest
+// and smallest up to 20 bits of their significands.
+__device__ __forceinline__ int high_key(double x) {
+  unsigned lo, hi;
+  sf64::halves(x, lo, hi);
+  return (int)(hi ^ (unsigned)(((int)hi >> 31) & 0x7fffffff));
+}
+// A lower bound in FP32 of the magnitude whose high half is h (0 for an
+// infinity or a NaN, which bound nothing).
+__device__ __forceinline__ float at_least(unsigned h) {
+  const unsigned f = (h - (896u << 20)) << 3;
+  return __uint_as_float(h < (897u << 20) || h >= 0x7ff00000u ? 0u
+                         : h >= (1150u << 20)                 ? 0x7f000000u
+                                                              : f);
+}
+
+struct side_limit {
+  long long key;
+  unsigned rare;
+};
+
+// What one side of the limiter allows a variable whose largest vertex
+// difference above u0 (UP, below u0 otherwise) may exceed the room that the
+// neighbours leave: the order key of min(1, (umax-u0)/du) or of
+// min(1, (umin-u0)/du).  g32 and E are the FP32 gradient and error bound of
+// cell_gradients: a vertex whose FP32 difference is more than 2 E below the
+// largest cannot be the largest, so the reference's arithmetic runs at the
+// largest one and at those within 2 E of it, with products and the quotient on
+// the integer pipes.  `rare` notes operands these leave to the hardware.
+template <int D, bool PRE, bool UP>
+__device__ __noinline__ side_limit limiter_side(const fvh_mesh_view &m, const tables &t,
+                                                const double *__restrict__ plane, int c0,
+                                                double u0, double g0, double g1, double g2,
+                                                float E) {
+  const double g[3] = {g0, g1, g2};
+  unsigned wide = 0, rare = 0;
+  float gf[D];
+#pragma unroll
+  for (int i = 0; i < D; ++i) gf[i] = UP ? truncated(g[i], wide) : -truncated(g[i], wide);
+  double x0[D];
+  if (!PRE) {
+#pragma unroll
+    for (int i = 0; i < D; ++i) x0[i] = m.cell_centroid[i][c0];
+  }
+  const int r0 = m.cell_vertex_offsets[c0], r1 = m.cell_vertex_offsets[c0 + 1];
+  auto estimate = [&](int rr) {
+    double dxv[D];
+    vertex_offset<D, PRE>(m, t, rr, x0, dxv);
+    float du = __fmul_rn(truncated(dxv[0], wide), gf[0]);
+#pragma unroll
+    for (int i = 1; i < D; ++i) du = __fmaf_rn(truncated(dxv[i], wide), gf[i], du);
+    return du;
+  };
+  long long kbest = 0;
+  auto exact = [&](int rr) {
+    double dxv[D];
+    vertex_offset<D, PRE>(m, t, rr, x0, dxv);
+    double u1 = u0;
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+      const flagged p = mul_call(dxv[i], g[i]);
+      rare |= p.rare;
+      u1 += p.q;
+    }
+    const long long kd = okey(u1 - u0);
+    kbest = (UP ? kbest < kd : kd < kbest) ? kd : kbest;
+  };
+  int best = r0;
+  float top = -1.f, next = -1.f;  // the two largest estimates (of those above 0)
+#pragma unroll 1
+  for (int rr = r0; rr < r1; ++rr) {
+    const float du = estimate(rr);
+    next = fmaxf(next, fminf(du, top));
+    if (du > top) {
+      top = du;
+      best = rr;
+    }
+  }
+  exact(best);
+  const float near = top - 2.0001f * E;
+  if (next >= near) {
+#pragma unroll 1
+    for (int rr = r0; rr < r1; ++rr)
+      if (rr != best && estimate(rr) >= near) exact(rr);
+  }
+  constexpr double tol = 1.e-9;
+  const long long one = okey(1.0);
+  if (UP ? !(kbest > okey(tol)) : !(kbest < okey(-tol))) return {one, rare};
+  long long kn = okey(u0);
+  const int q0 = m.cell_nbr_offsets[c0], q1 = m.cell_nbr_offsets[c0 + 1];
+#pragma unroll 4
+  for (int q = q0; q < q1; ++q) {
+    const long long k1 = okey(plane[m.cell_nbrs[q]]);
+    kn = (UP ? kn < k1 : k1 < kn) ? k1 : kn;
+  }
+  const double num = from_okey(kn) - u0;
+  if (UP ? !(okey(num) < kbest) : !(okey(num) > kbest)) return {one, rare};  // (see limiter_exact)
+  const flagged f = div_call(num, from_okey(kbest));
+  rare |= f.rare;
+  const long long kq = okey(f.q);
+  return {kq < one ? kq : one, rare};
+}
+
+// closed-form solve of the least-squares system from the sums b (tasks.h:238-262)
+template <class A>
+__device__ __forceinline__ void solve(A &ar, const double (&r)[4], const double (&b)[2],
+                                      double (&g)[2]) {
+  const auto a00 = ar.take(r[0]), a01 = ar.take(r[1]), a11 = ar.take(r[2]), den = ar.take(r[3]);
+  const auto b0 = ar.take(b[0]), b1 = ar.take(b[1]);
+  g[0] = ar.prod(ar.take(ar.prod(b0, a11) - ar.prod(b1, a01)), den);
+  g[1] = ar.prod(ar.take(ar.prod(b1, a00) - ar.prod(b0, a01)), den);
+}
+// 3D: products of the same two operands are formed once
+template <class A>
+__device__ __forceinline__ void solve(A &ar, const double (&r)[10], const double (&b)[3],
+                                      double (&g)[3]) {
+  const auto a00 = ar.take(r[0]), a01 = ar.take(r[1]), a02 = ar.take(r[2]), a11 = ar.take(r[3]),
+             a12 = ar.take(r[4]), a22 = ar.take(r[5]), den = ar.take(r[9]);
+  const auto b0 = ar.take(b[0]), b1 = ar.take(b[1]), b2 = ar.take(b[2]);
+  const double b1a12 = ar.prod(b1, a12), b2a11 = ar.prod(a11, b2);
+  const auto s = ar.take(ar.prod(b1, a22) - ar.prod(a12, b2));
+  const auto u = ar.take(ar.prod(b2, a01) - ar.prod(a02, b1));
+  g[0] = ar.prod(ar.take(ar.prod(b0, ar.take(r[6])) - ar.prod(a01, s) +
+                         ar.prod(a02, ar.take(b1a12 - b2a11))), den);
+  g[1] = ar.prod(ar.take(ar.prod(a00, s) - ar.prod(b0, ar.take(r[7])) + ar.prod(a02, u)), den);
+  g[2] = ar.prod(ar.take(ar.prod(a00, ar.take(b2a11 - b1a12)) - ar.prod(a01, u) +
+                         ar.prod(b0, ar.take(r[8]))), den);
+}
+
+// The limited gradients gu of cell c0 for the NK reconstructed variables from
+// k0 on (of d, v.., e, p, a); r: the cell's least-squares terms (read from the
+// table with PRE).  Each variable's gradient and limiter depend on that variable alone, so the
+// variables are taken in groups, each in its own pass over the neighbours.
+//
+// The limiter is decided in FP32 where FP32 can decide it: with every vertex
+// difference du within E of its FP32 estimate, a variable is not limited when
+// du <= tol, or du <= umax - u0 (RN(umax - u0) is the largest neighbour
+// difference, of which the key of the high half gives a lower bound), and
+// likewise below; phi is then 1 exactly.  The other variables take
+// limiter_exact.  In flows that are smooth or at rest up to rounding nearly
+// all are decided, which saves their vertex products and sums and the second
+// pass over the neighbours.
+template <int D, int NK, bool LIMIT, bool PRE, class A>
+__device__ __forceinline__ void cell_gradients(A &ar, const fvh_mesh_view &m,
+                                               const fvh_state_view &s, const tables &t, int c0,
+                                               int k0, const double (&r)[lsq_width<D>::value],
+                                               double (&gu)[NK][D]) {
+  double x0[D];
+  if (!PRE) {
+#pragma unroll
+    for (int i = 0; i < D; ++i) x0[i] = m.cell_centroid[i][c0];
+  }
+  const double *plane[NK];
+  double u0[NK], dudx[NK][D];
+  int kmax[NK], kmin[NK];
+#pragma unroll
+  for (int k = 0; k < NK; ++k) {
+    plane[k] = state_plane_at<D>(s, k0 + k);
+    u0[k] = plane[k][c0];
+    kmax[k] = kmin[k] = 0;
 #pragma unroll
     for (int j = 0; j < D; ++j) dudx[k][j] = 0;
+  }
   const int q0 = m.cell_nbr_offsets[c0], q1 = m.cell_nbr_offsets[c0 + 1];
-  #pragma unroll 1
-  for (int q = q0; q < q1; ++q) {
+  auto neighbour = [&](int q, bool first) {
     const int c1 = m.cell_nbrs[q];
-    double u1[NV];
-    load_values<D, K0, NK>(s, c1, u1);
-    double dx[D];
+    double du[NK], dx[D];
+#pragma unroll
+    for (int k = 0; k < NK; ++k) du[k] = plane[k][c1];
     if (PRE) {
       load_dx<D>(t.nbr_dx + (size_t)q * D, dx);
     } else {
 #pragma unroll
       for (int d = 0; d < D; ++d) dx[d] = m.cell_centroid[d][c1] - x0[d];
     }
-    double du[NV];
-    unsigned nonzero = 0;
+    bool same = true;
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      du[k] = u1[k] - u0[k];
-      nonzero |= (unsigned)!is_zero(du[k]);
+    for (int k = 0; k < NK; ++k) {
+      du[k] -= u0[k];
+      same = same && is_zero(du[k]);
+      if (LIMIT) {
+        const int key = high_key(du[k]);
+        kmax[k] = max(kmax[k], key);
+        kmin[k] = min(kmin[k], key);
+      }
     }
     // a neighbour equal to the cell in every variable adds (+-0) * dx = +-0 to
-    // each sum, which leaves it as it is (a sum that starts at +0 and adds
-    // nonzero terms is never -0): cells inside a uniform region skip it
-    if (nonzero) {
+    // each sum, which leaves it as it is: cells inside a uniform region skip it
+    if (same) return;
+    typename A::part px[D];
 #pragma unroll
-      for (int k = 0; k < NV; ++k)
+    for (int j = 0; j < D; ++j) px[j] = PRE ? ar.take_entry(dx[j]) : ar.take(dx[j]);
 #pragma unroll
-        for (int j = 0; j < D; ++j) dudx[k][j] += ar.mul(du[k], dx[j]);
-    }
-  }
-  double r[W];
-  if (PRE) {
+    for (int k = 0; k < NK; ++k) {
+      const auto pu = ar.take(du[k]);
 #pragma unroll
-    for (int k = 0; k < W; ++k) r[k] = t.lsq[(size_t)k * m.num_cells + c0];
-  } else {
-    lsq_matrix<D>(ar, m, c0, r);
-  }
-  if (D == 2) {
-    const double a00 = r[0], a01 = r[1], a11 = r[2], denom = r[3];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      gu[k][0] = ar.mul(ar.mul(dudx[k][0], a11) - ar.mul(dudx[k][1], a01), denom);
-      gu[k][D - 1] = ar.mul(ar.mul(dudx[k][1], a00) - ar.mul(dudx[k][0], a01), denom);
-    }
-  } else {
-    const double a00 = r[0], a01 = r[1], a02 = r[2], a11 = r[3], a12 = r[4], a22 = r[5];
-    const double min1 = r[6], min2 = r[7], min3 = r[W - 2], denom = r[W - 1];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      const double b0 = dudx[k][0], b1 = dudx[k][1], b2 = dudx[k][D - 1];
-      gu[k][0] = ar.mul(ar.mul(b0, min1) - ar.mul(a01, ar.mul(b1, a22) - ar.mul(a12, b2)) +
-                            ar.mul(a02, ar.mul(b1, a12) - ar.mul(a11, b2)),
-                        denom);
-      gu[k][1] = ar.mul(ar.mul(a00, ar.mul(b1, a22) - ar.mul(a12, b2)) - ar.mul(b0, min2) +
-                            ar.mul(a02, ar.mul(b2, a01) - ar.mul(a02, b1)),
-                        denom);
-      gu[k][D - 1] = ar.mul(ar.mul(a00, ar.mul(b2, a11) - ar.mul(a12, b1)) -
-                                ar.mul(a01, ar.mul(b2, a01) - ar.mul(a02, b1)) +
-                                ar.mul(b0, min3),
-                            denom);
-    }
-  }
-  if (LIMIT) {
-    // phi_k = min over vertices of (umax-u0)/du or (umin-u0)/du.  Correctly
-    // rounded division is monotone in the divisor, so for each variable only
-    // the largest du > tol and the smallest du < -tol can set the minimum; the
-    // result equals the reference's per-vertex minimum.
-    const long long ktol = okey(tol), kntol = okey(-tol);
-    long long kpos[NV], kneg[NV];
-    // a variable with a zero gradient has u1 == u0 at every vertex (to the
-    // sign of a zero, which the order keys do not see): no vertex limits it
-    bool graded[NV];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      kpos[k] = kneg[k] = 0;
-      graded[k] = false;
-#pragma unroll
-      for (int i = 0; i < D; ++i) graded[k] = graded[k] || !is_zero(gu[k][i]);
-    }
-    const int r0 = m.cell_vertex_offsets[c0], r1 = m.cell_vertex_offsets[c0 + 1];
-    #pragma unroll 1
-    for (int rr = r0; rr < r1; ++rr) {
-      double dxv[D];
-      if (PRE) {
-        load_dx<D>(t.vtx_dx + (size_t)rr * D, dxv);
-      } else {
-        const int vtx = m.cell_vertices[rr];
-#pragma unroll
-        for (int i = 0; i < D; ++i) dxv[i] = m.vertex_coord[i][vtx] - x0[i];
-      }
-#pragma unroll
-      for (int k = 0; k < NV; ++k) {
-        if (!graded[k]) continue;
-        double u1 = u0[k];
-#pragma unroll
-        for (int i = 0; i < D; ++i) u1 += ar.mul(dxv[i], gu[k][i]);
-        const long long kd = okey(u1 - u0[k]);
-        if (kd > ktol) kpos[k] = (kpos[k] < kd) ? kd : kpos[k];
-        else if (kd < kntol) kneg[k] = (kd < kneg[k]) ? kd : kneg[k];
+      for (int j = 0; j < D; ++j) {
+        if (first)
+          ar.add_first(dudx[k][j], pu, px[j]);
+        else
+          ar.add(dudx[k][j], pu, px[j]);
       }
     }
-    // the neighbour extrema umin / umax (tasks.h:232-236) are needed only for
-    // a variable some vertex value departs from by more than tol: they are
-    // taken then, in a second pass over the neighbours (whose values are
-    // still in cache), as order keys
+  };
+  if (q0 < q1) neighbour(q0, true);
+#pragma unroll 1
+  for (int q = q0 + 1; q < q1; ++q) neighbour(q, false);
+  {
+    double lsq[lsq_width<D>::value];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      long long kphi = okey(1.0);
-      if (kpos[k] > ktol || kneg[k] < kntol) {
-        const double *plane = state_plane<D>(s, K0 + k);
-        long long kmin = okey(u0[k]), kmax = kmin;
-        #pragma unroll 1
-        for (int q = q0; q < q1; ++q) {
-          const long long k1 = okey(plane[m.cell_nbrs[q]]);
-          kmin = (k1 < kmin) ? k1 : kmin;  // std::min(u1, umin)
-          kmax = (kmax < k1) ? k1 : kmax;  // std::max(u1, umax)
-        }
-        // RN(N / du) >= 1 exactly when |N| >= |du| (N and du of one sign, du
-        // normal), so the quotient is formed only when it can lower phi below 1
-        if (kpos[k] > ktol) {
-          const double num = from_okey(kmax) - u0[k];
-          if (okey(num) < kpos[k]) {
-            const long long kq = okey(ar.quo(num, from_okey(kpos[k])));
-            kphi = (kq < kphi) ? kq : kphi;
-          }
-        }
-        if (kneg[k] < kntol) {
-          const double num = from_okey(kmin) - u0[k];
-          if (okey(num) > kneg[k]) {
-            const long long kq = okey(ar.quo(num, from_okey(kneg[k])));
-            kphi = (kq < kphi) ? kq : kphi;
-          }
-        }
+    for (int w = 0; w < lsq_width<D>::value; ++w)
+      lsq[w] = PRE ? t.lsq[(size_t)w * m.num_cells + c0] : r[w];
+#pragma unroll
+    for (int k = 0; k < NK; ++k) solve(ar, lsq, dudx[k], gu[k]);
+  }
+  if (!LIMIT) return;
+  float gf[NK][D], top[NK], low[NK], reach[D];
+  unsigned wide[NK], far = 0;
+#pragma unroll
+  for (int i = 0; i < D; ++i) reach[i] = 0.f;
+#pragma unroll
+  for (int k = 0; k < NK; ++k) {
+    wide[k] = 0;
+    top[k] = low[k] = 0.f;
+#pragma unroll
+    for (int i = 0; i < D; ++i) gf[k][i] = truncated(gu[k][i], wide[k]);
+  }
+  const int r0 = m.cell_vertex_offsets[c0], r1 = m.cell_vertex_offsets[c0 + 1];
+#pragma unroll 1
+  for (int rr = r0; rr < r1; ++rr) {
+    double dxv[D];
+    float f[D];
+    vertex_offset<D, PRE>(m, t, rr, x0, dxv);
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+      f[i] = truncated(dxv[i], far);
+      reach[i] = fmaxf(reach[i], fabsf(f[i]));
+    }
+#pragma unroll
+    for (int k = 0; k < NK; ++k) {
+      float du = __fmul_rn(f[0], gf[k][0]);
+#pragma unroll
+      for (int i = 1; i < D; ++i) du = __fmaf_rn(f[i], gf[k][i], du);
+      top[k] = fmaxf(top[k], du);
+      low[k] = fminf(low[k], du);
+    }
+  }
+  // E: truncating g and dx and the FP32 roundings move sum |dx g| by less than
+  // 2^-21 of itself; values below 2^-60 taken as zero; the reference's own
+  // roundings about u0 by less than 2^-50 |u0|.  Each term is taken double.
+  float tiny = 1e-30f;
+#pragma unroll
+  for (int i = 0; i < D; ++i) tiny = __fmaf_rn(reach[i], 0x1p-59f, tiny);
+#pragma unroll
+  for (int k = 0; k < NK; ++k) {
+    float E = __fmaf_rn(fabsf(truncated(u0[k], wide[k])), 0x1p-49f, tiny);
+#pragma unroll
+    for (int i = 0; i < D; ++i)
+      E = __fmaf_rn(__fmaf_rn(reach[i], 0x1p-20f, 0x1p-59f), fabsf(gf[k][i]), E);
+    const float up = top[k] + E, down = E - low[k];
+    const float room = at_least((unsigned)kmax[k]);
+    const float floor = at_least((unsigned)~kmin[k] & 0x7fffffffu);
+    constexpr float tol = 0.9999e-9f;
+    const bool free_up = up <= tol || up <= room, free_down = down <= tol || down <= floor;
+    unsigned odd = wide[k] | far;
+    if (free_up && free_down && !odd) continue;
+    long long kphi = okey(1.0);
+    const double *gk = gu[k];
+    if (!odd) {
+      if (!free_up) {
+        const side_limit l = limiter_side<D, PRE, true>(m, t, plane[k], c0, u0[k], gk[0], gk[1],
+                                                        gk[D - 1], E);
+        kphi = l.key;
+        odd = l.rare;
+      }
+      if (!free_down) {
+        const side_limit l = limiter_side<D, PRE, false>(m, t, plane[k], c0, u0[k], gk[0], gk[1],
+                                                         gk[D - 1], E);
+        kphi = l.key < kphi ? l.key : kphi;
+        odd |= l.rare;
       }
       kphi = (kphi < 0) ? 0 : kphi;  // std::max(phi, 0)
-      if (kphi != okey(1.0)) {
-        const double phi = from_okey(kphi);
+    }
+    if (odd) kphi = okey(limiter_exact<D, PRE>(m, t, plane[k], c0, u0[k], gk[0], gk[1], gk[D - 1]));
+    if (kphi != okey(1.0)) {
+      const auto phi = ar.take(from_okey(kphi));
 #pragma unroll
-        for (int i = 0; i < D; ++i) gu[k][i] = ar.mul(gu[k][i], phi);
-      }
+      for (int i = 0; i < D; ++i) gu[k][i] = ar.prod(ar.take(gu[k][i]), phi);
     }
   }
 }
 
-template <int D, int K0, int NK>
-__device__ __forceinline__ void store_gradients(const fvh_gradient_view &g, int c0,
+template <int D, int NK>
+__device__ __forceinline__ void store_gradients(const fvh_gradient_view &g, int c0, int k0,
                                                 const double (&gu)[NK][D]) {
 #pragma unroll
   for (int k = 0; k < NK; ++k)
 #pragma unroll
-    for (int i = 0; i < D; ++i) grad_plane<D>(g, K0 + k, i)[c0] = gu[k][i];
+    for (int i = 0; i < D; ++i) grad_planes_at<D>(g, k0 + k)[i][c0] = gu[k][i];
 }
 
 // the FP64 redo of a cell whose operands left the integer-pipe range, out of
 // line (it is rare and would otherwise double the kernel's code)
-template <int D, int K0, int NK, bool LIMIT, bool PRE>
+template <int D, int NK, bool LIMIT, bool PRE>
 __device__ __noinline__ void gradient_group_hw(const fvh_mesh_view &m, const fvh_state_view &s,
                                                const fvh_gradient_view &g, const tables &t,
-                                               int c0) {
-  double gu[NK][D];
+                                               int c0, int k0) {
+  double gu[NK][D], r[lsq_width<D>::value];
   arith_hw hw;
-  cell_gradients<D, K0, NK, LIMIT, PRE>(hw, m, s, t, c0, gu);
-  store_gradients<D, K0, NK>(g, c0, gu);
+  if (!PRE) lsq_matrix<D>(hw, m, c0, r);
+  cell_gradients<D, NK, LIMIT, PRE>(hw, m, s, t, c0, k0, r, gu);
+  store_gradients<D, NK>(g, c0, k0, gu);
 }
 
-// the gradients of variables K0 .. K0+NK-1 of cell c0, stored
-template <int D, int K0, int NK, bool LIMIT, bool PRE>
+// the gradients of NK variables from k0 on of cell c0, stored
+template <int D, int NK, bool LIMIT, bool PRE>
 __device__ __forceinline__ void gradient_group(const fvh_mesh_view &m, const fvh_state_view &s,
                                                const fvh_gradient_view &g, const tables &t,
-                                               int c0) {
+                                               int c0, int k0,
+                                               const double (&r)[lsq_width<D>::value],
+                                               unsigned rare) {
   double gu[NK][D];
   arith_opt ar;
-  cell_gradients<D, K0, NK, LIMIT, PRE>(ar, m, s, t, c0, gu);
+  ar.rare = rare;
+  cell_gradients<D, NK, LIMIT, PRE>(ar, m, s, t, c0, k0, r, gu);
   if (ar.rare) {
-    gradient_group_hw<D, K0, NK, LIMIT, PRE>(m, s, g, t, c0);
+    gradient_group_hw<D, NK, LIMIT, PRE>(m, s, g, t, c0, k0);
     return;
   }
-  store_gradients<D, K0, NK>(g, c0, gu);
+  store_gradients<D, NK>(g, c0, k0, gu);
 }
 
-// Blocks of 128 per SM the kernels are compiled for.  2D (1024^2 workload, ms
-// per step): fluxes 7 (72 registers) 1.493 against 1.502 with 6 and 1.542
-// with 8; gradients 10 (48 registers, variables in pairs, below) 1.572
-// against 1.582 with 8; update 10 (48 registers) 1.487 against 1.502 with
-// the compiler's choice (66 registers) and 1.493 with 8.  3D (96^3 hex):
-// gradients and fluxes 5 blocks (96 registers) 5.68 against 5.92 with 3 and
-// 4 and 5.88 with 4 and 5; update the compiler's choice.
+// Blocks of 128 per SM the kernels are compiled for.  2D (1024^2 four-quadrant
+// workload, 4 steps): fluxes 7 (72 registers) 4.88 ms against 4.98 with 6 and
+// 4.89 with 8; gradients 9 4.78 against 4.83 with 7 and 4.78 with 10 (a flow
+// with waves everywhere 5.84, 5.87 and 5.85); update 10 (48 registers).  3D
+// (80^3 hex, 2 steps): fluxes 5 (96 registers) 0.311 ms a launch against 0.320
+// with 4 and 0.329 with 6; gradients 7 4.30 ms against 4.35 with 6 and 4.42
+// with 5; update the compiler's choice.
 template <int D>
 constexpr int min_blocks() { return D == 2 ? 7 : 5; }
 template <int D>
-constexpr int grad_min_blocks() { return D == 2 ? 10 : 5; }
+constexpr int grad_min_blocks() { return D == 2 ? 9 : 7; }
 template <int D>
 constexpr int update_min_blocks() { return D == 2 ? 10 : 1; }
-// Variables per neighbour pass of the gradients.  Each variable's gradient
-// and limiter depend on that variable alone, so the variables can be taken in
-// groups, each in its own pass over the neighbours (the neighbours' values
-// are re-read, mostly from L1/L2): fewer live sums, more warps.  2D in pairs
-// (d vx, vy e, p a): 1.572 ms per step against 1.755 with all six in one pass
-// and 1.592 in threes; 3D in groups of four (d v, then e p a): 5.30 against
-// 5.58 in threes (6 blocks) and 5.30 in pairs.
-template <int D>
-__host__ __device__ constexpr int grad_split() { return D == 2 ? 2 : D + 1; }
-
-// the variables K0 .. NV-1 in groups of G, each group in its own pass
-template <int D, int K0, int G, bool LIMIT, bool PRE>
-__device__ __forceinline__ void gradient_groups(const fvh_mesh_view &m, const fvh_state_view &s,
-                                                const fvh_gradient_view &g, const tables &t,
-                                                int c0) {
-  constexpr int NV = D + 4, NK = (NV - K0 < G) ? NV - K0 : G;
-  gradient_group<D, K0, NK, LIMIT, PRE>(m, s, g, t, c0);
-  if constexpr (K0 + NK < NV) gradient_groups<D, K0 + NK, G, LIMIT, PRE>(m, s, g, t, c0);
-}
+// Variables per neighbour pass of the gradients: two, in 3D the last one alone
+// (fewer live sums, more warps; the offsets x_nbr - x_c are taken apart once
+// for both).  1024^2, 4 steps: 4.83 ms against 4.77 one by one and 5.09 in
+// threes, with waves everywhere 5.99 against 6.13 and 6.11; 3D 80^3, 2 steps:
+// 4.23 against 4.40 one by one and 5.03 in fours.
+constexpr int kGradGroup = 2;
 
 template <int D, bool LIMIT, bool PRE>
 __global__ void __launch_bounds__(kCellThreads, grad_min_blocks<D>())
-gradients_kernel(const fvh_mesh_view m, const fvh_state_view s, const fvh_gradient_view g,
-                 const tables t) {
+gradients_kernel(const __grid_constant__ fvh_mesh_view m, const __grid_constant__ fvh_state_view s,
+                 const __grid_constant__ fvh_gradient_view g, const __grid_constant__ tables t) {
   const int c0 = blockIdx.x * blockDim.x + threadIdx.x;
   if (c0 >= m.num_cells) return;
-  gradient_groups<D, 0, grad_split<D>(), LIMIT, PRE>(m, s, g, t, c0);
+  constexpr int NV = D + 4, G = kGradGroup;
+  double r[lsq_width<D>::value];
+  arith_opt ar;
+  if (!PRE) lsq_matrix<D>(ar, m, c0, r);
+#pragma unroll 1
+  for (int k0 = 0; k0 + G <= NV; k0 += G) gradient_group<D, G, LIMIT, PRE>(m, s, g, t, c0, k0, r, ar.rare);
+  if constexpr (NV % G != 0)
+    gradient_group<D, NV % G, LIMIT, PRE>(m, s, g, t, c0, NV - NV % G, r, ar.rare);
 }
 
 // ---------------------------------------------------------------------------
 // face fluxes (tasks.h:385-464)
 // ---------------------------------------------------------------------------
-template <int D, bool SECOND, class A>
+template <int D, bool SECOND, bool PRE, class A>
 __device__ __forceinline__ prim<D> reconstruct(A &ar, const fvh_state_view &s,
                                                const fvh_gradient_view &g, int c,
                                                const double *dx, bool swap) {
@@ -824,12 +1119,15 @@ __device__ __forceinline__ prim<D> reconstruct(A &ar, const fvh_state_view &s,
     if (nonzero | !plain) {
 #pragma unroll
       for (int i = 0; i < D; ++i) {
-        w.d += ar.mul(dx[i], gd[i]);
+        // dx is taken apart once for all of its products
+        const auto px = PRE ? ar.take_entry(dx[i]) : ar.take(dx[i]);
+        auto step = [&](double &u, double gr) { u += ar.prod(px, ar.take(gr)); };
+        step(w.d, gd[i]);
 #pragma unroll
-        for (int d = 0; d < D; ++d) w.v[d] += ar.mul(dx[i], gv[d][i]);
-        w.p += ar.mul(dx[i], gpp[i]);
-        w.e += ar.mul(dx[i], gee[i]);
-        w.a += ar.mul(dx[i], ga[i]);
+        for (int d = 0; d < D; ++d) step(w.v[d], gv[d][i]);
+        step(w.p, gpp[i]);
+        step(w.e, gee[i]);
+        step(w.a, ga[i]);
       }
     }
   }
@@ -859,10 +1157,10 @@ __device__ __forceinline__ void face_flux(A &ar, const fvh_mesh_view &m,
   for (int i = 0; i < D; ++i) n[i] = m.face_normal[i][f];
   double dx[D] = {};
   if (SECOND) face_offset<D, PRE>(m, face_dx, f, 0, cc.x, dx);
-  const prim<D> wl = reconstruct<D, SECOND>(ar, s, g, cc.x, dx, swap);
+  const prim<D> wl = reconstruct<D, SECOND, PRE>(ar, s, g, cc.x, dx, swap);
   if (cc.y >= 0) {
     if (SECOND) face_offset<D, PRE>(m, face_dx, f, 1, cc.y, dx);
-    const prim<D> wr = reconstruct<D, SECOND>(ar, s, g, cc.y, dx, swap);
+    const prim<D> wr = reconstruct<D, SECOND, PRE>(ar, s, g, cc.y, dx, swap);
     if (KIND == FVH_FLUX_RUSANOV)
       rusanov<D>(ar, wl, wr, n, F);
     else if (KIND == FVH_FLUX_HLLC)
@@ -870,7 +1168,7 @@ __device__ __forceinline__ void face_flux(A &ar, const fvh_mesh_view &m,
     else
       hlle<D>(ar, wl, wr, n, F);
   } else if (outflow) {
-    phys_flux<D>(ar, wl, n, F);
+    phys_flux<D>(ar, wl, n, dot<D>(ar, wl.v, n), total_energy<D>(ar, wl), F);
   } else {
     F[0] = 0;
 #pragma unroll
@@ -900,8 +1198,9 @@ __device__ __noinline__ void face_flux_hw(const fvh_mesh_view &m, const fvh_stat
 
 template <int D, int KIND, bool SECOND, bool PRE>
 __global__ void __launch_bounds__(kFaceThreads, min_blocks<D>())
-fluxes_kernel(const fvh_mesh_view m, const fvh_state_view s, const fvh_gradient_view g,
-              const fvh_flux_view fl, int swap, int outflow, const double *__restrict__ face_dx) {
+fluxes_kernel(const __grid_constant__ fvh_mesh_view m, const __grid_constant__ fvh_state_view s,
+              const __grid_constant__ fvh_gradient_view g, const __grid_constant__ fvh_flux_view fl,
+              int swap, int outflow, const double *__restrict__ face_dx) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= m.num_faces) return;
   const int2 cc = reinterpret_cast<const int2 *>(m.face_cells)[f];
@@ -923,6 +1222,13 @@ fluxes_kernel(const fvh_mesh_view m, const fvh_state_view s, const fvh_gradient_
 // ---------------------------------------------------------------------------
 // gather + conservative update + EOS (tasks.h:589-659)
 // ---------------------------------------------------------------------------
+// 0 - F or 0 + F: F with that sign, +0 for a zero
+__device__ __forceinline__ double signed_flux(double F, bool minus) {
+  unsigned lo, hi;
+  sf64::halves(F, lo, hi);
+  return sf64::join(lo, sf64::is_zero(lo, hi) ? 0u : hi ^ (minus ? 0x80000000u : 0u));
+}
+
 // the new state of cell c: w = (d, v.., e, p, T, a^2)
 // gm1 = gamma - 1 and ggm1 = gamma * (gamma - 1), rounded once on the host
 // exactly as the reference rounds them per cell (euler_eqns.h / ideal_gas.h)
@@ -943,17 +1249,17 @@ __device__ __forceinline__ void cell_update(A &ar, const fvh_mesh_view &m,
 #pragma unroll
     for (int i = 0; i < D; ++i) F[1 + i] = fl.momentum[i][f];
     F[D + 1] = fl.energy[f];
-    // the update kernel's FP64 pipe is its bound (83 %, ALU 43 %): the sums of
-    // the first two faces run on the integer pipe (2D step 1.516 -> 1.488 ms);
-    // a - b is a + (-b) exactly
-    if (q - q0 < 2) {
-      if (sf >= 0) {
+    // the first sum, 0 -+ F, is F with its sign
+    if (q == q0) {
 #pragma unroll
-        for (int k = 0; k < D + 2; ++k) du[k] = add_call(du[k], -F[k]);
-      } else {
+      for (int k = 0; k < D + 2; ++k) du[k] = signed_flux(F[k], sf >= 0);
+      continue;
+    }
+    // the update kernel's FP64 pipe is its bound: the next face's sums run on
+    // the integer pipe; a - b is a + (-b) exactly
+    if (q == q0 + 1) {
 #pragma unroll
-        for (int k = 0; k < D + 2; ++k) du[k] = add_call(du[k], F[k]);
-      }
+      for (int k = 0; k < D + 2; ++k) du[k] = add_call(du[k], sf >= 0 ? -F[k] : F[k]);
       continue;
     }
     if (sf >= 0) {
@@ -1117,7 +1423,7 @@ size_t table_doubles(int dim, int64_t nc, int64_t nf, int64_t nnz_cf, int64_t nn
   // each table starts on a 256-byte boundary (32 doubles)
   auto up = [](int64_t x) { return (x + 31) / 32 * 32; };
   return (size_t)(up(w * nc) + up(nnz_cf) + up(dim * nnz_nb) + up(dim * nnz_cv) +
-                  up(2 * dim * nf));
+                  up(2 * dim * nf) + 32);
 }
 
 template <int D>
@@ -1129,15 +1435,26 @@ cudaError_t build_tables(const fvh_mesh_view &m, double *base, int64_t nnz_cf,
   double *nbr_dx = slot_dx + up(nnz_cf);
   double *vtx_dx = nbr_dx + up(D * nnz_nb);
   double *face_dx = vtx_dx + up(D * nnz_cv);
+  unsigned *d_odd = reinterpret_cast<unsigned *>(face_dx + up(2 * D * (int64_t)m.num_faces));
+  unsigned odd = 0;
+  cudaError_t e = cudaMemset(d_odd, 0, sizeof(unsigned));
+  if (e != cudaSuccess) return e;
   const int th = 128;
-  cell_tables_kernel<D><<<(m.num_cells + th - 1) / th, th>>>(m, lsq, slot_dx, nbr_dx, vtx_dx);
-  face_tables_kernel<D><<<(m.num_faces + th - 1) / th, th>>>(m, face_dx);
+  cell_tables_kernel<D><<<(m.num_cells + th - 1) / th, th>>>(m, lsq, slot_dx, nbr_dx, vtx_dx,
+                                                             d_odd);
+  face_tables_kernel<D><<<(m.num_faces + th - 1) / th, th>>>(m, face_dx, d_odd);
+  e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpy(&odd, d_odd, sizeof(unsigned), cudaMemcpyDeviceToHost);
+  if (e != cudaSuccess) return e;
   t->lsq = lsq;
   t->slot_dx = slot_dx;
   t->nbr_dx = nbr_dx;
   t->vtx_dx = vtx_dx;
   t->face_dx = face_dx;
-  return cudaGetLastError();
+  // the kernels take these offsets unchecked: a mesh with others computes
+  // them on the fly
+  if (odd) t->nbr_dx = t->face_dx = nullptr;
+  return cudaSuccess;
 }
 
 template <int D, bool SECOND, bool PRE>

@@ -86,16 +86,23 @@ struct parts {
   bool zero;
 };
 
-// Takes x apart; `rare` collects whether it is neither moderate nor a zero.
-__device__ __forceinline__ parts take(double x, unsigned &rare) {
+// Takes a moderate value or a zero apart.
+__device__ __forceinline__ parts take_plain(double x) {
   unsigned lo, hi;
   halves(x, lo, hi);
   parts p;
   p.lo = lo;
   p.m = (hi & 0xfffffu) | 0x100000u;
   p.se = hi & 0xfff00000u;
+  p.zero = ((hi & 0x7fffffffu) | lo) == 0u;
+  return p;
+}
+// Takes x apart; `rare` collects whether it is neither moderate nor a zero.
+__device__ __forceinline__ parts take(double x, unsigned &rare) {
+  const parts p = take_plain(x);
+  unsigned lo, hi;
+  halves(x, lo, hi);
   const unsigned h = hi & 0x7fffffffu;
-  p.zero = (h | lo) == 0u;
   rare |= (unsigned)!((h - (523u << 20) < (1001u << 20)) | p.zero);
   return p;
 }

@@ -46,6 +46,7 @@ struct fvh_solver {
   fvh::plain::tables tab;          // views into `tables`
   double *scalars = nullptr;       // [0] soln time, [1] dt, [2..] dt partials
   fvh_device_status *status = nullptr;
+  unsigned long long *dt_maximum = nullptr;  // FP64 form: plain::next_dt::maximum
   double *host_scalars = nullptr;  // pinned: soln time
   fvh_device_status *host_status = nullptr;
   fvh::mixed::workspace *mixed = nullptr;
@@ -223,6 +224,8 @@ fvh_status fvh_solver_create(const fvh_mesh_view *mesh, const fvh_params *params
     cudaError_t e = cudaSuccess;
     if (params->precision == FVH_PRECISION_FP64) {
       e = cudaMalloc(&s->work, sizeof(double) * (ng * nc + (size_t)(D + 2) * nf));
+      // zero gradients, which a first-order solver keeps
+      if (e == cudaSuccess) e = cudaMemset(s->work, 0, sizeof(double) * ng * nc);
       if (e == cudaSuccess) {
         double *b = s->work;
         for (int i = 0; i < D; ++i, b += nc) s->grads.density[i] = b;
@@ -256,7 +259,10 @@ fvh_status fvh_solver_create(const fvh_mesh_view *mesh, const fvh_params *params
     }
     if (e == cudaSuccess)
       e = cudaMalloc(&s->scalars, sizeof(double) * 2 + fvh_time_step_workspace_bytes(mesh->num_cells));
-    if (e == cudaSuccess) e = cudaMalloc(&s->status, sizeof(fvh_device_status));
+    // the status word and the FP64 form's carried CFL maximum
+    if (e == cudaSuccess) e = cudaMalloc(&s->status, sizeof(fvh_device_status) + 8);
+    if (e == cudaSuccess) s->dt_maximum = s->status + 1;
+    if (e == cudaSuccess) e = cudaMemset(s->dt_maximum, 0, 8);
     if (e == cudaSuccess) e = cudaMallocHost(&s->host_scalars, sizeof(double) * 2);
     if (e == cudaSuccess) e = cudaMallocHost(&s->host_status, sizeof(fvh_device_status));
     if (e == cudaSuccess) e = cudaMemset(s->scalars, 0, sizeof(double) * 2);
@@ -281,34 +287,49 @@ static fvh_status solver_step_enqueue(fvh_solver *s, const fvh_state_view *state
   if (p.precision == FVH_PRECISION_MIXED)
     return from_cuda(fvh::mixed::step(s->mixed, m, p, *state, t, dt, partial,
                                       dt_blocks(m.num_cells), s->status, st, mark, s->shape, f));
-  const fvh_stream_t fs = reinterpret_cast<fvh_stream_t>(st);
   const int nb = dt_blocks(m.num_cells);
-  fvh_status r = from_cuda(
-      m.dim == 2 ? fvh::plain::launch_dt<2>(m, *state, p, t, dt, partial, nb, s->status, st,
-                                            s->tab.slot_dx, f.src)
-                 : fvh::plain::launch_dt<3>(m, *state, p, t, dt, partial, nb, s->status, st,
-                                            s->tab.slot_dx, f.src));
-  mark("dt");
+  fvh::plain::next_dt nd;
+  nd.maximum = s->dt_maximum;
+  nd.cfl = p.cfl;
+  nd.final_time = p.final_time;
+  nd.soln_time = t;
+  nd.dt = dt;
+  nd.status = s->status;
+  const fvh::plain::next_dt none;
+  fvh_status r = FVH_OK;
+  if (f.pack_first) {
+    r = from_cuda(m.dim == 2 ? fvh::plain::launch_dt<2>(m, *state, p, t, dt, partial, nb, s->status,
+                                                        st, s->tab.slot_dx, f.src, nd.maximum)
+                             : fvh::plain::launch_dt<3>(m, *state, p, t, dt, partial, nb, s->status,
+                                                        st, s->tab.slot_dx, f.src, nd.maximum));
+    mark("dt");
+  }
   for (int stage = 0; stage < 2 && r == FVH_OK; ++stage) {
-    if (p.order == 1)
-      r = fvh_evaluate_gradients(&m, state, &s->grads, &p, fs);
-    else
-      r = from_cuda(m.dim == 2
-                        ? fvh::plain::launch_gradients<2>(m, *state, s->grads, p, st, s->tab)
-                        : fvh::plain::launch_gradients<3>(m, *state, s->grads, p, st, s->tab));
-    mark("gradients");
+    // a step that follows another of its run forms dt in its first kernel
+    const fvh::plain::next_dt &first = stage == 0 && !f.pack_first ? nd : none;
+    if (p.order != 1) {  // (first order: the gradients stay zero as created)
+      r = from_cuda(m.dim == 2 ? fvh::plain::launch_gradients<2>(m, *state, s->grads, p, st,
+                                                                 s->tab, first)
+                               : fvh::plain::launch_gradients<3>(m, *state, s->grads, p, st,
+                                                                 s->tab, first));
+      mark("gradients");
+    }
     if (r == FVH_OK)
-      r = from_cuda(m.dim == 2
-                        ? fvh::plain::launch_fluxes<2>(m, *state, s->grads, s->flux, p, st, s->tab)
-                        : fvh::plain::launch_fluxes<3>(m, *state, s->grads, s->flux, p, st, s->tab));
+      r = from_cuda(m.dim == 2 ? fvh::plain::launch_fluxes<2>(m, *state, s->grads, s->flux, p, st,
+                                                              s->tab, first)
+                               : fvh::plain::launch_fluxes<3>(m, *state, s->grads, s->flux, p, st,
+                                                              s->tab, first));
     mark("fluxes");
-    // the last stage of the step may also write the new state to f.out
+    // the last stage of the step may also write the new state to f.out and
+    // take the next step's CFL maximum
     const fvh_state_view *out = stage == 1 ? f.out : nullptr;
+    const fvh::plain::next_dt &next = stage == 1 && f.write_next ? nd : none;
     if (r == FVH_OK)
-      r = from_cuda(m.dim == 2 ? fvh::plain::launch_update<2>(m, p, dt, 0.5, s->flux, *state, t,
-                                                              s->status, st, out)
-                               : fvh::plain::launch_update<3>(m, p, dt, 0.5, s->flux, *state, t,
-                                                              s->status, st, out));
+      r = from_cuda(m.dim == 2
+                        ? fvh::plain::launch_update<2>(m, p, dt, 0.5, s->flux, *state, t, s->status,
+                                                       st, out, s->tab.slot_dx, next)
+                        : fvh::plain::launch_update<3>(m, p, dt, 0.5, s->flux, *state, t, s->status,
+                                                       st, out, s->tab.slot_dx, next));
     mark("update");
   }
   return r;
@@ -479,8 +500,8 @@ fvh_status fvh_debug_sf64(int32_t op, const double *a, const double *b, int64_t 
 
 int64_t fvh_solver_launches_per_run(const fvh_solver *s, int64_t nsteps) {
   if (!s || nsteps <= 0) return 0;
-  if (s->params.precision != FVH_PRECISION_MIXED)
-    return nsteps * fvh_solver_launches_per_step(s);
+  if (s->params.precision != FVH_PRECISION_MIXED)  // dt (two kernels) in the first step only
+    return 2 + nsteps * (fvh_solver_launches_per_step(s) - 2);
   int64_t total = 0;
   for (int64_t k = 0; k < nsteps && k < 2; ++k)  // the first step and one of the rest
     total += fvh::mixed::launches_per_step(s->params, s->shape, chunk_flags(k, nsteps),
@@ -497,10 +518,8 @@ int32_t fvh_solver_launches_per_step(const fvh_solver *s) {
   if (s->params.precision == FVH_PRECISION_MIXED)
     return fvh::mixed::launches_per_step(s->params, s->shape, {},
                                          fvh::mixed::colours(s->mixed));
-  // dt (partial + final) + per stage: gradients (or D*(D+4) memsets), fluxes, update
-  const int D = s->mesh.dim;
-  const int grad = s->params.order == 1 ? D * (D + 4) : 1;
-  return 2 + 2 * (grad + 2);
+  // dt (partial + final) + per stage: gradients (none at first order), fluxes, update
+  return 2 + 2 * ((s->params.order == 1 ? 0 : 1) + 2);
 }
 
 namespace {
@@ -574,7 +593,6 @@ fvh_status fvh_solver_profile(fvh_solver *s, const fvh_state_view *state, int32_
 // (stream, state) into a CUDA graph and replayed.
 static fvh_status solver_step_flags(fvh_solver *s, const fvh_state_view *state, cudaStream_t st,
                                     fvh::mixed::step_flags f) {
-  if (s->params.precision != FVH_PRECISION_MIXED) f = fvh::mixed::step_flags();
   if (st == nullptr) return solver_step_enqueue(s, state, st, {}, f);
   if (s->graph_stream != st || std::memcmp(&s->graph_state, state, sizeof(*state)) != 0) {
     drop_graphs(s);

@@ -66,33 +66,50 @@ template <int D>
 cudaError_t build_tables(const fvh_mesh_view &m, double *base, int64_t nnz_cf,
                          int64_t nnz_nb, int64_t nnz_cv, tables *t);
 
+// dt carried from one step of a run to the next: the last update of a step
+// takes the CFL maximum of the new state into *maximum (as the bits of a
+// positive double, cleared when dt is formed), and the first kernel of the next
+// step forms dt from it.  With maximum null neither happens.
+struct next_dt {
+  unsigned long long *maximum = nullptr;
+  double cfl = 0, final_time = 0;
+  const double *soln_time = nullptr;
+  double *dt = nullptr;
+  fvh_device_status *status = nullptr;
+};
+
 template <int D>
 cudaError_t launch_dt(const fvh_mesh_view &m, const fvh_state_view &s,
                       const fvh_params &p, const double *soln_time, double *dt,
                       double *partial, int nblocks, fvh_device_status *status,
                       cudaStream_t st, const double *slot_dx = nullptr,
-                      const fvh_state_view *src = nullptr);
+                      const fvh_state_view *src = nullptr,
+                      unsigned long long *maximum = nullptr);
 template <int D>
 cudaError_t launch_gradients(const fvh_mesh_view &m, const fvh_state_view &s,
                              const fvh_gradient_view &g, const fvh_params &p,
-                             cudaStream_t st, const tables &t = tables());
+                             cudaStream_t st, const tables &t = tables(),
+                             const next_dt &nd = next_dt());
 template <int D>
 cudaError_t launch_fluxes(const fvh_mesh_view &m, const fvh_state_view &s,
                           const fvh_gradient_view &g, const fvh_flux_view &fl,
-                          const fvh_params &p, cudaStream_t st, const tables &t = tables());
+                          const fvh_params &p, cudaStream_t st, const tables &t = tables(),
+                          const next_dt &nd = next_dt());
 // Diagnostic: out[i] = a[i] op b[i] for op 0 mul, 1 add, 2 sub, 3 div on the
 // integer pipes (fvh_sf64.cuh), 4..7 the same with the FP64 instructions,
 // 8 / 9 the optimistic mul / div with their FP64 redo.
 cudaError_t debug_sf64(int op, const double *a, const double *b, int64_t n, double *out,
                        cudaStream_t st);
 // out (optional): a second copy of the new state, e.g. host-mapped planes of
-// a caller that holds its state in host memory
+// a caller that holds its state in host memory; with nd.maximum the CFL maximum
+// of the new state is taken too (slot_dx: tables::slot_dx)
 template <int D>
 cudaError_t launch_update(const fvh_mesh_view &m, const fvh_params &p, const double *dt,
                           double factor, const fvh_flux_view &fl,
                           const fvh_state_view &s, double *soln_time,
                           fvh_device_status *status, cudaStream_t st,
-                          const fvh_state_view *out = nullptr);
+                          const fvh_state_view *out = nullptr,
+                          const double *slot_dx = nullptr, const next_dt &nd = next_dt());
 }  // namespace plain
 
 }  // namespace fvh

@@ -41,6 +41,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "flecsale_gb300.h"
 #include "fvh_kernels.h"
@@ -48,6 +49,20 @@
 
 namespace fvh {
 namespace plain {
+
+// Few cells or faces leave most of the chip idle and a kernel's time is one
+// thread's chain of loads and operations.  The FP64 instructions are then the
+// shorter chain (their pipe is shared by few warps), small blocks reach more SMs
+// and unrolled loops load ahead.  Where the lines lie: a step with such gradients
+// takes 58 us at 64^2 against 60 with the integer forms one variable a thread
+// and 68 in pairs, at 112^2 71, 68 and 75; in 3D at 16^3 107, 115 and 132, at
+// 20^3 139, 130 and 152.  Without tables the four tasks take 85 us against 116
+// at 64^2, 111 and 118 at 128^2, 168 and 148 at 200^2.  Fluxes: 11 us a launch against
+// 12.5 with 2,112 faces, both 12.3 with 18,600.  Update: 11 against 11.5 us with
+// 1,024 cells, 19 against 15 with 44,000.
+constexpr int kFewThreads = 64;
+constexpr int kFewCells = 6144, kFewCellsNoTables = 16384, kFewFaces = 10000;
+constexpr int kFewUpdateCells = 20000;
 
 // Products and quotients in out-of-line calls (a call costs a few
 // instructions; inlining them everywhere made the kernels too large for the
@@ -76,6 +91,7 @@ __device__ __noinline__ double add_call(double a, double b) { return sf64::add(a
 // Products and quotients of one unit of work: on the integer pipes, noting
 // any operand they leave to the hardware ...
 struct arith_opt {
+  static constexpr bool wide_issue = true;  // many warps: skip what adds nothing
   using part = sf64::parts;
   unsigned rare = 0;
   // an operand of several products is taken apart once
@@ -118,6 +134,7 @@ struct arith_opt {
 };
 // ... and with the FP64 instructions (the evaluation kept when `rare`)
 struct arith_hw {
+  static constexpr bool wide_issue = false;  // few warps: independent loads, no branches
   static constexpr unsigned rare = 0;
   using part = double;
   __device__ __forceinline__ part take(double x) { return x; }
@@ -382,16 +399,14 @@ __device__ __forceinline__ double from_okey(long long k) {
 // mesh by the same division.
 // ---------------------------------------------------------------------------
 template <int D, bool PRE, class A>
-__device__ __forceinline__ double cell_dt_inv(A &ar, const fvh_mesh_view &m,
-                                              const fvh_state_view &s, int c,
+__device__ __forceinline__ double cell_dt_inv(A &ar, const fvh_mesh_view &m, int c,
+                                              const double *v, double a,
                                               const double *__restrict__ slot_dx) {
-  double v[D];
-#pragma unroll
-  for (int i = 0; i < D; ++i) v[i] = s.velocity[i][c];
-  const double a = s.sound_speed[c];
   const double vol = PRE ? 0.0 : m.cell_volume[c];
   double dt_inv = 0;
   const int q0 = m.cell_face_offsets[c], q1 = m.cell_face_offsets[c + 1];
+  constexpr int U = A::wide_issue ? 1 : 4;
+#pragma unroll U
   for (int q = q0; q < q1; ++q) {
     int f = m.cell_faces[q];
     f = f < 0 ? ~f : f;
@@ -404,6 +419,17 @@ __device__ __forceinline__ double cell_dt_inv(A &ar, const fvh_mesh_view &m,
     dt_inv = smax(dti, dt_inv);
   }
   return dt_inv;
+}
+
+// the same, evaluated again with the FP64 instructions where an operand is rare
+template <int D, bool PRE>
+__device__ __forceinline__ double cell_dt_inv_any(const fvh_mesh_view &m, int c, const double *v,
+                                                  double a, const double *__restrict__ slot_dx) {
+  arith_opt ar;
+  const double r = cell_dt_inv<D, PRE>(ar, m, c, v, a, slot_dx);
+  if (!ar.rare) return r;
+  arith_hw hw;
+  return cell_dt_inv<D, PRE>(hw, m, c, v, a, slot_dx);
 }
 
 // With has_src the state is read from src (e.g. host-mapped planes of a caller
@@ -424,37 +450,58 @@ dt_partial_kernel(const fvh_mesh_view m, const fvh_state_view s, double *partial
       s.pressure[c] = src.pressure[c];
       s.sound_speed[c] = src.sound_speed[c];
     }
-    arith_opt ar;
-    double cell = cell_dt_inv<D, PRE>(ar, m, s, c, slot_dx);
-    if (ar.rare) {
-      arith_hw hw;
-      cell = cell_dt_inv<D, PRE>(hw, m, s, c, slot_dx);
-    }
+    double v[D];
+#pragma unroll
+    for (int i = 0; i < D; ++i) v[i] = s.velocity[i][c];
     // the reference's running maximum over cells and faces, taken cell by
     // cell (a maximum of maxima: the same value)
-    dt_inv = smax(cell, dt_inv);
+    dt_inv = smax(cell_dt_inv_any<D, PRE>(m, c, v, s.sound_speed[c], slot_dx), dt_inv);
   }
   dt_inv = block_max(dt_inv);
   if (threadIdx.x == 0) partial[blockIdx.x] = dt_inv;
 }
 
+// dt = min(CFL / maximum, t_f - t)
+__device__ __forceinline__ void write_dt(double dt_inv, double cfl, double final_time,
+                                         const double *soln_time, double *dt_out,
+                                         fvh_device_status *status) {
+  const double max_dt = final_time - soln_time[0];
+  if (le0(dt_inv)) {
+    atomicMin(status, status_key(0, FVH_ERR_INFINITE_DT));
+    dt_out[0] = 0;
+  } else {
+    double time_step = __ddiv_rn(1, dt_inv);
+    time_step = __dmul_rn(time_step, cfl);
+    dt_out[0] = smin(time_step, max_dt);
+  }
+}
+
 __global__ void __launch_bounds__(kDtThreads)
-dt_final_kernel(const double *partial, int nblocks, fvh_params p,
-                const double *soln_time, double *dt_out, fvh_device_status *status) {
+dt_final_kernel(const double *partial, int nblocks, fvh_params p, const double *soln_time,
+                double *dt_out, fvh_device_status *status, unsigned long long *maximum) {
   double dt_inv = 0;
   for (int i = threadIdx.x; i < nblocks; i += blockDim.x) dt_inv = smax(partial[i], dt_inv);
   dt_inv = block_max(dt_inv);
   if (threadIdx.x == 0) {
-    const double max_dt = p.final_time - soln_time[0];
-    if (le0(dt_inv)) {
-      atomicMin(status, status_key(0, FVH_ERR_INFINITE_DT));
-      dt_out[0] = 0;
-    } else {
-      double time_step = __ddiv_rn(1, dt_inv);
-      time_step = __dmul_rn(time_step, p.cfl);
-      dt_out[0] = smin(time_step, max_dt);
-    }
+    write_dt(dt_inv, p.cfl, p.final_time, soln_time, dt_out, status);
+    if (maximum) *maximum = 0ull;  // (a run that failed half-way may have left one)
   }
+}
+
+// Inside a run the last update of a step also takes the CFL maximum of the new
+// state (next_dt::maximum, the order of positive doubles is that of their
+// bits), and the first kernel of the following step, which does not read dt,
+// turns it into dt and clears it.
+__device__ __forceinline__ void finish_dt(const next_dt &nd) {
+  if (!nd.maximum || blockIdx.x != 0 || blockIdx.y != 0 || threadIdx.x != 0) return;
+  const double dt_inv = __longlong_as_double((long long)*nd.maximum);
+  *nd.maximum = 0ull;
+  write_dt(dt_inv, nd.cfl, nd.final_time, nd.soln_time, nd.dt, nd.status);
+}
+__device__ __forceinline__ void add_to_maximum(const next_dt &nd, double dt_inv) {
+  dt_inv = block_max(dt_inv);
+  if (threadIdx.x == 0 && lt(0.0, dt_inv))
+    atomicMax(nd.maximum, (unsigned long long)__double_as_longlong(dt_inv));
 }
 
 // ---------------------------------------------------------------------------
@@ -897,7 +944,7 @@ __device__ __forceinline__ void cell_gradients(A &ar, const fvh_mesh_view &m,
     }
     // a neighbour equal to the cell in every variable adds (+-0) * dx = +-0 to
     // each sum, which leaves it as it is: cells inside a uniform region skip it
-    if (same) return;
+    if (A::wide_issue && same) return;
     typename A::part px[D];
 #pragma unroll
     for (int j = 0; j < D; ++j) px[j] = PRE ? ar.take_entry(dx[j]) : ar.take(dx[j]);
@@ -914,7 +961,8 @@ __device__ __forceinline__ void cell_gradients(A &ar, const fvh_mesh_view &m,
     }
   };
   if (q0 < q1) neighbour(q0, true);
-#pragma unroll 1
+  constexpr int U = A::wide_issue ? 1 : 4;
+#pragma unroll U
   for (int q = q0 + 1; q < q1; ++q) neighbour(q, false);
   {
     double lsq[lsq_width<D>::value];
@@ -937,7 +985,7 @@ __device__ __forceinline__ void cell_gradients(A &ar, const fvh_mesh_view &m,
     for (int i = 0; i < D; ++i) gf[k][i] = truncated(gu[k][i], wide[k]);
   }
   const int r0 = m.cell_vertex_offsets[c0], r1 = m.cell_vertex_offsets[c0 + 1];
-#pragma unroll 1
+#pragma unroll U
   for (int rr = r0; rr < r1; ++rr) {
     double dxv[D];
     float f[D];
@@ -1010,17 +1058,27 @@ __device__ __forceinline__ void store_gradients(const fvh_gradient_view &g, int 
     for (int i = 0; i < D; ++i) grad_planes_at<D>(g, k0 + k)[i][c0] = gu[k][i];
 }
 
+// the gradients of NK variables from k0 on of cell c0 with the FP64
+// instructions, stored
+template <int D, int NK, bool LIMIT, bool PRE>
+__device__ __forceinline__ void gradient_group_fp64(const fvh_mesh_view &m,
+                                                    const fvh_state_view &s,
+                                                    const fvh_gradient_view &g, const tables &t,
+                                                    int c0, int k0) {
+  double gu[NK][D], r[lsq_width<D>::value];
+  arith_hw hw;
+  if (!PRE) lsq_matrix<D>(hw, m, c0, r);
+  cell_gradients<D, NK, LIMIT, PRE>(hw, m, s, t, c0, k0, r, gu);
+  store_gradients<D, NK>(g, c0, k0, gu);
+}
+
 // the FP64 redo of a cell whose operands left the integer-pipe range, out of
 // line (it is rare and would otherwise double the kernel's code)
 template <int D, int NK, bool LIMIT, bool PRE>
 __device__ __noinline__ void gradient_group_hw(const fvh_mesh_view &m, const fvh_state_view &s,
                                                const fvh_gradient_view &g, const tables &t,
                                                int c0, int k0) {
-  double gu[NK][D], r[lsq_width<D>::value];
-  arith_hw hw;
-  if (!PRE) lsq_matrix<D>(hw, m, c0, r);
-  cell_gradients<D, NK, LIMIT, PRE>(hw, m, s, t, c0, k0, r, gu);
-  store_gradients<D, NK>(g, c0, k0, gu);
+  gradient_group_fp64<D, NK, LIMIT, PRE>(m, s, g, t, c0, k0);
 }
 
 // the gradients of NK variables from k0 on of cell c0, stored
@@ -1043,38 +1101,59 @@ __device__ __forceinline__ void gradient_group(const fvh_mesh_view &m, const fvh
 
 // Blocks of 128 per SM the kernels are compiled for.  2D (1024^2 four-quadrant
 // workload, 4 steps): fluxes 7 (72 registers) 4.88 ms against 4.98 with 6 and
-// 4.89 with 8; gradients 9 4.78 against 4.83 with 7 and 4.78 with 10 (a flow
-// with waves everywhere 5.84, 5.87 and 5.85); update 10 (48 registers).  3D
+// 4.89 with 8; gradients 10 4.74 against 4.77 with 9 and 4.81 with 8 (a flow
+// with waves everywhere 5.78, 5.79 and 5.84); update 10 (48 registers).  3D
 // (80^3 hex, 2 steps): fluxes 5 (96 registers) 0.311 ms a launch against 0.320
-// with 4 and 0.329 with 6; gradients 7 4.30 ms against 4.35 with 6 and 4.42
-// with 5; update the compiler's choice.
+// with 4 and 0.329 with 6; gradients 8 4.02 ms against 4.08 with 7 and 4.18
+// with 6; update the compiler's choice.  Gradients without tables: 3D 6.
 template <int D>
 constexpr int min_blocks() { return D == 2 ? 7 : 5; }
-template <int D>
-constexpr int grad_min_blocks() { return D == 2 ? 9 : 7; }
+template <int D, bool PRE>
+constexpr int grad_min_blocks() { return PRE ? (D == 2 ? 10 : 8) : (D == 2 ? 7 : 6); }
 template <int D>
 constexpr int update_min_blocks() { return D == 2 ? 10 : 1; }
-// Variables per neighbour pass of the gradients: two, in 3D the last one alone
-// (fewer live sums, more warps; the offsets x_nbr - x_c are taken apart once
-// for both).  1024^2, 4 steps: 4.83 ms against 4.77 one by one and 5.09 in
-// threes, with waves everywhere 5.99 against 6.13 and 6.11; 3D 80^3, 2 steps:
-// 4.23 against 4.40 one by one and 5.03 in fours.
-constexpr int kGradGroup = 2;
+// Variables of a cell per thread (blockIdx.y: which).  In pairs the offsets
+// x_nbr - x_c are read and taken apart once for both; one by one gives twice the
+// threads, which wins until the chip is full: 10 steps at 360^2 2.58 ms against
+// 2.68 in pairs, at 512^2 4.71 and 4.71, at 1024^2 (4 steps) 4.97 and 4.74; in
+// 3D 5 steps 2.93 against 2.94 at 44^3, 4.24 against 4.08 at 50^3.  All of a
+// cell's variables in one thread: 4.28 ms against 4.08 (80^3, 2 steps); threes
+// 4.51.  Without tables a thread takes all of them, as it builds the
+// least-squares matrix itself.
+constexpr int kSingleCells2D = 262144, kSingleCells3D = 92160;
 
-template <int D, bool LIMIT, bool PRE>
-__global__ void __launch_bounds__(kCellThreads, grad_min_blocks<D>())
+template <int D, bool LIMIT, bool PRE, int G>
+__global__ void __launch_bounds__(kCellThreads, grad_min_blocks<D, PRE>())
 gradients_kernel(const __grid_constant__ fvh_mesh_view m, const __grid_constant__ fvh_state_view s,
-                 const __grid_constant__ fvh_gradient_view g, const __grid_constant__ tables t) {
+                 const __grid_constant__ fvh_gradient_view g, const __grid_constant__ tables t,
+                 const __grid_constant__ next_dt nd) {
+  finish_dt(nd);
   const int c0 = blockIdx.x * blockDim.x + threadIdx.x;
   if (c0 >= m.num_cells) return;
-  constexpr int NV = D + 4, G = kGradGroup;
+  constexpr int NV = D + 4, R = NV % G;
   double r[lsq_width<D>::value];
   arith_opt ar;
+  int k0 = PRE ? blockIdx.y * G : 0;
   if (!PRE) lsq_matrix<D>(ar, m, c0, r);
 #pragma unroll 1
-  for (int k0 = 0; k0 + G <= NV; k0 += G) gradient_group<D, G, LIMIT, PRE>(m, s, g, t, c0, k0, r, ar.rare);
-  if constexpr (NV % G != 0)
-    gradient_group<D, NV % G, LIMIT, PRE>(m, s, g, t, c0, NV - NV % G, r, ar.rare);
+  for (; k0 + G <= NV; k0 += PRE ? NV + 1 : G)
+    gradient_group<D, G, LIMIT, PRE>(m, s, g, t, c0, k0, r, ar.rare);
+  if constexpr (R != 0)
+    if (k0 == NV - R) gradient_group<D, R, LIMIT, PRE>(m, s, g, t, c0, k0, r, ar.rare);
+}
+
+// Few cells (kFewCells): one variable of one cell per thread (blockIdx.y), with
+// the FP64 instructions.
+template <int D, bool LIMIT, bool PRE>
+__global__ void __launch_bounds__(kFewThreads)
+gradients_few_kernel(const __grid_constant__ fvh_mesh_view m,
+                     const __grid_constant__ fvh_state_view s,
+                     const __grid_constant__ fvh_gradient_view g,
+                     const __grid_constant__ tables t, const __grid_constant__ next_dt nd) {
+  finish_dt(nd);
+  const int c0 = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c0 >= m.num_cells) return;
+  gradient_group_fp64<D, 1, LIMIT, PRE>(m, s, g, t, c0, blockIdx.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -1116,7 +1195,7 @@ __device__ __forceinline__ prim<D> reconstruct(A &ar, const fvh_state_view &s,
     unsigned plain = (unsigned)(ordinary(w.d) & ordinary(w.p) & ordinary(w.e) & ordinary(w.a));
 #pragma unroll
     for (int d = 0; d < D; ++d) plain &= (unsigned)ordinary(w.v[d]);
-    if (nonzero | !plain) {
+    if (!A::wide_issue || (nonzero | !plain)) {
 #pragma unroll
       for (int i = 0; i < D; ++i) {
         // dx is taken apart once for all of its products
@@ -1180,6 +1259,14 @@ __device__ __forceinline__ void face_flux(A &ar, const fvh_mesh_view &m,
   for (int k = 0; k < D + 2; ++k) F[k] = __dmul_rn(F[k], area);
 }
 
+template <int D>
+__device__ __forceinline__ void store_flux(const fvh_flux_view &fl, int f, const double *F) {
+  fl.mass[f] = F[0];
+#pragma unroll
+  for (int i = 0; i < D; ++i) fl.momentum[i][f] = F[1 + i];
+  fl.energy[f] = F[D + 1];
+}
+
 // the FP64 redo of a face whose operands left the integer-pipe range, out of
 // line
 template <int D, int KIND, bool SECOND, bool PRE>
@@ -1190,33 +1277,44 @@ __device__ __noinline__ void face_flux_hw(const fvh_mesh_view &m, const fvh_stat
   double F[D + 2];
   arith_hw hw;
   face_flux<D, KIND, SECOND, PRE>(hw, m, s, g, f, cc, swap != 0, outflow != 0, face_dx, F);
-  fl.mass[f] = F[0];
-#pragma unroll
-  for (int i = 0; i < D; ++i) fl.momentum[i][f] = F[1 + i];
-  fl.energy[f] = F[D + 1];
+  store_flux<D>(fl, f, F);
 }
 
 template <int D, int KIND, bool SECOND, bool PRE>
 __global__ void __launch_bounds__(kFaceThreads, min_blocks<D>())
 fluxes_kernel(const __grid_constant__ fvh_mesh_view m, const __grid_constant__ fvh_state_view s,
               const __grid_constant__ fvh_gradient_view g, const __grid_constant__ fvh_flux_view fl,
-              int swap, int outflow, const double *__restrict__ face_dx) {
+              int swap, int outflow, const double *__restrict__ face_dx,
+              const __grid_constant__ next_dt nd) {
+  if (!SECOND) finish_dt(nd);  // (first order has no gradients)
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= m.num_faces) return;
   const int2 cc = reinterpret_cast<const int2 *>(m.face_cells)[f];
   double F[D + 2];
-  {
-    arith_opt ar;
-    face_flux<D, KIND, SECOND, PRE>(ar, m, s, g, f, cc, swap != 0, outflow != 0, face_dx, F);
-    if (ar.rare) {
-      face_flux_hw<D, KIND, SECOND, PRE>(m, s, g, fl, f, cc, swap, outflow, face_dx);
-      return;
-    }
+  arith_opt ar;
+  face_flux<D, KIND, SECOND, PRE>(ar, m, s, g, f, cc, swap != 0, outflow != 0, face_dx, F);
+  if (ar.rare) {
+    face_flux_hw<D, KIND, SECOND, PRE>(m, s, g, fl, f, cc, swap, outflow, face_dx);
+    return;
   }
-  fl.mass[f] = F[0];
-#pragma unroll
-  for (int i = 0; i < D; ++i) fl.momentum[i][f] = F[1 + i];
-  fl.energy[f] = F[D + 1];
+  store_flux<D>(fl, f, F);
+}
+
+// Few faces (kFewFaces): with the FP64 instructions.
+template <int D, int KIND, bool SECOND, bool PRE>
+__global__ void __launch_bounds__(kFewThreads)
+fluxes_few_kernel(const __grid_constant__ fvh_mesh_view m, const __grid_constant__ fvh_state_view s,
+                  const __grid_constant__ fvh_gradient_view g,
+                  const __grid_constant__ fvh_flux_view fl, int swap, int outflow,
+                  const double *__restrict__ face_dx, const __grid_constant__ next_dt nd) {
+  if (!SECOND) finish_dt(nd);
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= m.num_faces) return;
+  double F[D + 2];
+  arith_hw hw;
+  face_flux<D, KIND, SECOND, PRE>(hw, m, s, g, f, reinterpret_cast<const int2 *>(m.face_cells)[f],
+                                  swap != 0, outflow != 0, face_dx, F);
+  store_flux<D>(fl, f, F);
 }
 
 // ---------------------------------------------------------------------------
@@ -1241,6 +1339,8 @@ __device__ __forceinline__ void cell_update(A &ar, const fvh_mesh_view &m,
 #pragma unroll
   for (int k = 0; k < D + 2; ++k) du[k] = 0;
   const int q0 = m.cell_face_offsets[c], q1 = m.cell_face_offsets[c + 1];
+  constexpr int U = A::wide_issue ? 2 : 4;
+#pragma unroll U
   for (int q = q0; q < q1; ++q) {
     const int sf = m.cell_faces[q];
     const int f = sf < 0 ? ~sf : sf;
@@ -1257,7 +1357,7 @@ __device__ __forceinline__ void cell_update(A &ar, const fvh_mesh_view &m,
     }
     // the update kernel's FP64 pipe is its bound: the next face's sums run on
     // the integer pipe; a - b is a + (-b) exactly
-    if (q == q0 + 1) {
+    if (A::wide_issue && q == q0 + 1) {
 #pragma unroll
       for (int k = 0; k < D + 2; ++k) du[k] = add_call(du[k], sf >= 0 ? -F[k] : F[k]);
       continue;
@@ -1293,43 +1393,56 @@ __device__ __forceinline__ void cell_update(A &ar, const fvh_mesh_view &m,
   w[D + 4] = ar.mul(ggm1, e);                 // a^2; its root is taken once
 }
 
-template <int D>
-__global__ void __launch_bounds__(kCellThreads, update_min_blocks<D>())
-update_kernel(const fvh_mesh_view m, const fvh_flux_view fl, const fvh_state_view s,
-              const double *dt, double factor, double gm1, double ggm1, double cv,
-              double *soln_time, fvh_device_status *status, const fvh_state_view out,
-              int has_out) {
+// FEW (kFewUpdateCells): with the FP64 instructions.  NEXT: the last update of a step that
+// another one follows; slot_dx the table of V / A.
+template <int D, bool FEW, bool NEXT>
+__global__ void __launch_bounds__(FEW ? kFewThreads : kCellThreads, FEW ? 1 : update_min_blocks<D>())
+update_kernel(const __grid_constant__ fvh_mesh_view m, const __grid_constant__ fvh_flux_view fl,
+              const __grid_constant__ fvh_state_view s, const double *dt, double factor, double gm1,
+              double ggm1, double cv, double *soln_time, fvh_device_status *status,
+              const __grid_constant__ fvh_state_view out, int has_out,
+              const double *__restrict__ slot_dx, const __grid_constant__ next_dt nd) {
   const double delta_t = __dmul_rn(dt[0], factor);
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c == 0) soln_time[0] = 0.0 + soln_time[0] + delta_t;
-  if (c >= m.num_cells) return;
-  double w[D + 5];
-  {
+  if (!NEXT && c >= m.num_cells) return;
+  double dt_inv = 0;
+  if (!NEXT || c < m.num_cells) {
+    double w[D + 5];
     arith_opt ar;
-    cell_update<D>(ar, m, fl, s, c, delta_t, gm1, ggm1, cv, w);
-    if (ar.rare) {
+    if (!FEW) cell_update<D>(ar, m, fl, s, c, delta_t, gm1, ggm1, cv, w);
+    if (FEW || ar.rare) {
       arith_hw hw;
       cell_update<D>(hw, m, fl, s, c, delta_t, gm1, ggm1, cv, w);
     }
-  }
-  const double a = sqrt(w[D + 4]);
-  s.density[c] = w[0];
+    const double a = sqrt(w[D + 4]);
+    s.density[c] = w[0];
 #pragma unroll
-  for (int i = 0; i < D; ++i) s.velocity[i][c] = w[1 + i];
-  s.internal_energy[c] = w[D + 1];
-  s.pressure[c] = w[D + 2];
-  s.temperature[c] = w[D + 3];
-  s.sound_speed[c] = a;
-  if (has_out) {
-    out.density[c] = w[0];
+    for (int i = 0; i < D; ++i) s.velocity[i][c] = w[1 + i];
+    s.internal_energy[c] = w[D + 1];
+    s.pressure[c] = w[D + 2];
+    s.temperature[c] = w[D + 3];
+    s.sound_speed[c] = a;
+    if (has_out) {
+      out.density[c] = w[0];
 #pragma unroll
-    for (int i = 0; i < D; ++i) out.velocity[i][c] = w[1 + i];
-    out.internal_energy[c] = w[D + 1];
-    out.pressure[c] = w[D + 2];
-    out.temperature[c] = w[D + 3];
-    out.sound_speed[c] = a;
+      for (int i = 0; i < D; ++i) out.velocity[i][c] = w[1 + i];
+      out.internal_energy[c] = w[D + 1];
+      out.pressure[c] = w[D + 2];
+      out.temperature[c] = w[D + 3];
+      out.sound_speed[c] = a;
+    }
+    if (lt0(w[D + 1]) || lt0(w[0])) atomicMin(status, status_key(c, FVH_ERR_NEGATIVE_STATE));
+    if (NEXT) {
+      if (FEW) {
+        arith_hw hw;
+        dt_inv = cell_dt_inv<D, true>(hw, m, c, w + 1, a, slot_dx);
+      } else {
+        dt_inv = cell_dt_inv_any<D, true>(m, c, w + 1, a, slot_dx);
+      }
+    }
   }
-  if (lt0(w[D + 1]) || lt0(w[0])) atomicMin(status, status_key(c, FVH_ERR_NEGATIVE_STATE));
+  if (NEXT) add_to_maximum(nd, dt_inv);
 }
 
 // ---------------------------------------------------------------------------
@@ -1381,11 +1494,14 @@ cudaError_t debug_sf64(int op, const double *a, const double *b, int64_t n, doub
 // ---------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------
+static int blocks_of(int n, int threads) { return (n + threads - 1) / threads; }
+
 template <int D>
 cudaError_t launch_dt(const fvh_mesh_view &m, const fvh_state_view &s,
                       const fvh_params &p, const double *soln_time, double *dt,
                       double *partial, int nblocks, fvh_device_status *status,
-                      cudaStream_t st, const double *slot_dx, const fvh_state_view *src) {
+                      cudaStream_t st, const double *slot_dx, const fvh_state_view *src,
+                      unsigned long long *maximum) {
   const fvh_state_view from = src ? *src : s;
   if (slot_dx)
     dt_partial_kernel<D, true><<<nblocks, kDtThreads, 0, st>>>(m, s, partial, slot_dx, from,
@@ -1393,27 +1509,35 @@ cudaError_t launch_dt(const fvh_mesh_view &m, const fvh_state_view &s,
   else
     dt_partial_kernel<D, false><<<nblocks, kDtThreads, 0, st>>>(m, s, partial, nullptr, from,
                                                                 src ? 1 : 0);
-  dt_final_kernel<<<1, kDtThreads, 0, st>>>(partial, nblocks, p, soln_time, dt, status);
+  dt_final_kernel<<<1, kDtThreads, 0, st>>>(partial, nblocks, p, soln_time, dt, status, maximum);
   return cudaGetLastError();
 }
 
 template <int D>
 cudaError_t launch_gradients(const fvh_mesh_view &m, const fvh_state_view &s,
                              const fvh_gradient_view &g, const fvh_params &p,
-                             cudaStream_t st, const tables &t) {
-  const int nb = (m.num_cells + kCellThreads - 1) / kCellThreads;
-  const bool lim = p.limiter != FVH_LIMITER_NONE;
-  if (t.lsq && t.nbr_dx && t.vtx_dx) {
-    if (lim)
-      gradients_kernel<D, true, true><<<nb, kCellThreads, 0, st>>>(m, s, g, t);
+                             cudaStream_t st, const tables &t, const next_dt &nd) {
+  const bool lim = p.limiter != FVH_LIMITER_NONE, pre = t.lsq && t.nbr_dx && t.vtx_dx;
+  if (m.num_cells <= (pre ? kFewCells : kFewCellsNoTables)) {
+    const dim3 grid(blocks_of(m.num_cells, kFewThreads), D + 4);
+    auto go = [&](auto kernel) { kernel<<<grid, kFewThreads, 0, st>>>(m, s, g, t, nd); };
+    if (pre)
+      lim ? go(gradients_few_kernel<D, true, true>) : go(gradients_few_kernel<D, false, true>);
     else
-      gradients_kernel<D, false, true><<<nb, kCellThreads, 0, st>>>(m, s, g, t);
-  } else {
-    if (lim)
-      gradients_kernel<D, true, false><<<nb, kCellThreads, 0, st>>>(m, s, g, t);
-    else
-      gradients_kernel<D, false, false><<<nb, kCellThreads, 0, st>>>(m, s, g, t);
+      lim ? go(gradients_few_kernel<D, true, false>) : go(gradients_few_kernel<D, false, false>);
+    return cudaGetLastError();
   }
+  auto go = [&](auto kernel, int groups) {
+    const dim3 grid(blocks_of(m.num_cells, kCellThreads), groups);
+    kernel<<<grid, kCellThreads, 0, st>>>(m, s, g, t, nd);
+  };
+  const int pairs = blocks_of(D + 4, 2);
+  if (!pre)
+    lim ? go(gradients_kernel<D, true, false, 2>, 1) : go(gradients_kernel<D, false, false, 2>, 1);
+  else if (m.num_cells <= (D == 2 ? kSingleCells2D : kSingleCells3D))
+    lim ? go(gradients_kernel<D, true, true, 1>, D + 4) : go(gradients_kernel<D, false, true, 1>, D + 4);
+  else
+    lim ? go(gradients_kernel<D, true, true, 2>, pairs) : go(gradients_kernel<D, false, true, 2>, pairs);
   return cudaGetLastError();
 }
 
@@ -1460,29 +1584,38 @@ cudaError_t build_tables(const fvh_mesh_view &m, double *base, int64_t nnz_cf,
 template <int D, bool SECOND, bool PRE>
 static void launch_fluxes_kind(const fvh_mesh_view &m, const fvh_state_view &s,
                                const fvh_gradient_view &g, const fvh_flux_view &fl,
-                               const fvh_params &p, cudaStream_t st, const double *face_dx) {
-  const int nb = (m.num_faces + kFaceThreads - 1) / kFaceThreads;
+                               const fvh_params &p, cudaStream_t st, const double *face_dx,
+                               const next_dt &nd) {
+  auto go = [&](auto kernel, int threads) {
+    kernel<<<blocks_of(m.num_faces, threads), threads, 0, st>>>(m, s, g, fl, p.recon_swap_ep,
+                                                               p.boundary, face_dx, nd);
+  };
+  auto kind = [&](auto k) {
+    constexpr int KIND = decltype(k)::value;
+    if (m.num_faces <= kFewFaces)
+      go(fluxes_few_kernel<D, KIND, SECOND, PRE>, kFewThreads);
+    else
+      go(fluxes_kernel<D, KIND, SECOND, PRE>, kFaceThreads);
+  };
   if (p.flux_kind == FVH_FLUX_RUSANOV)
-    fluxes_kernel<D, FVH_FLUX_RUSANOV, SECOND, PRE><<<nb, kFaceThreads, 0, st>>>(
-        m, s, g, fl, p.recon_swap_ep, p.boundary, face_dx);
+    kind(std::integral_constant<int, FVH_FLUX_RUSANOV>());
   else if (p.flux_kind == FVH_FLUX_HLLC)
-    fluxes_kernel<D, FVH_FLUX_HLLC, SECOND, PRE><<<nb, kFaceThreads, 0, st>>>(
-        m, s, g, fl, p.recon_swap_ep, p.boundary, face_dx);
+    kind(std::integral_constant<int, FVH_FLUX_HLLC>());
   else
-    fluxes_kernel<D, FVH_FLUX_HLLE, SECOND, PRE><<<nb, kFaceThreads, 0, st>>>(
-        m, s, g, fl, p.recon_swap_ep, p.boundary, face_dx);
+    kind(std::integral_constant<int, FVH_FLUX_HLLE>());
 }
 
 template <int D>
 cudaError_t launch_fluxes(const fvh_mesh_view &m, const fvh_state_view &s,
                           const fvh_gradient_view &g, const fvh_flux_view &fl,
-                          const fvh_params &p, cudaStream_t st, const tables &t) {
+                          const fvh_params &p, cudaStream_t st, const tables &t,
+                          const next_dt &nd) {
   if (p.order == 1)
-    launch_fluxes_kind<D, false, false>(m, s, g, fl, p, st, nullptr);
+    launch_fluxes_kind<D, false, false>(m, s, g, fl, p, st, nullptr, nd);
   else if (t.face_dx)
-    launch_fluxes_kind<D, true, true>(m, s, g, fl, p, st, t.face_dx);
+    launch_fluxes_kind<D, true, true>(m, s, g, fl, p, st, t.face_dx, nd);
   else
-    launch_fluxes_kind<D, true, false>(m, s, g, fl, p, st, nullptr);
+    launch_fluxes_kind<D, true, false>(m, s, g, fl, p, st, nullptr, nd);
   return cudaGetLastError();
 }
 
@@ -1491,14 +1624,22 @@ cudaError_t launch_update(const fvh_mesh_view &m, const fvh_params &p, const dou
                           double factor, const fvh_flux_view &fl,
                           const fvh_state_view &s, double *soln_time,
                           fvh_device_status *status, cudaStream_t st,
-                          const fvh_state_view *out) {
-  const int nb = (m.num_cells + kCellThreads - 1) / kCellThreads;
+                          const fvh_state_view *out, const double *slot_dx, const next_dt &nd) {
   // the same two roundings as (gamma - 1.0) and gamma * (gamma - 1.0) per cell
   const double gamma = p.gamma;
   const double gm1 = gamma - 1.0;
   const double ggm1 = gamma * gm1;
-  update_kernel<D><<<nb, kCellThreads, 0, st>>>(m, fl, s, dt, factor, gm1, ggm1, p.cv,
-                                                soln_time, status, out ? *out : s, out ? 1 : 0);
+  auto go = [&](auto kernel, int threads) {
+    kernel<<<blocks_of(m.num_cells, threads), threads, 0, st>>>(
+        m, fl, s, dt, factor, gm1, ggm1, p.cv, soln_time, status, out ? *out : s, out ? 1 : 0,
+        slot_dx, nd);
+  };
+  if (m.num_cells <= kFewUpdateCells)
+    nd.maximum ? go(update_kernel<D, true, true>, kFewThreads)
+               : go(update_kernel<D, true, false>, kFewThreads);
+  else
+    nd.maximum ? go(update_kernel<D, false, true>, kCellThreads)
+               : go(update_kernel<D, false, false>, kCellThreads);
   return cudaGetLastError();
 }
 
@@ -1506,20 +1647,23 @@ cudaError_t launch_update(const fvh_mesh_view &m, const fvh_params &p, const dou
   template cudaError_t launch_dt<D>(const fvh_mesh_view &, const fvh_state_view &,     \
                                     const fvh_params &, const double *, double *,      \
                                     double *, int, fvh_device_status *, cudaStream_t,  \
-                                    const double *, const fvh_state_view *);           \
+                                    const double *, const fvh_state_view *,            \
+                                    unsigned long long *);                             \
   template cudaError_t launch_gradients<D>(const fvh_mesh_view &, const fvh_state_view &, \
                                            const fvh_gradient_view &, const fvh_params &, \
-                                           cudaStream_t, const tables &);              \
+                                           cudaStream_t, const tables &, const next_dt &);              \
   template cudaError_t build_tables<D>(const fvh_mesh_view &, double *, int64_t, int64_t, \
                                        int64_t, tables *);                             \
   template cudaError_t launch_fluxes<D>(const fvh_mesh_view &, const fvh_state_view &, \
                                         const fvh_gradient_view &, const fvh_flux_view &, \
-                                        const fvh_params &, cudaStream_t, const tables &); \
+                                        const fvh_params &, cudaStream_t, const tables &, \
+                                        const next_dt &); \
   template cudaError_t launch_update<D>(const fvh_mesh_view &, const fvh_params &,     \
                                         const double *, double, const fvh_flux_view &, \
                                         const fvh_state_view &, double *,              \
                                         fvh_device_status *, cudaStream_t,             \
-                                        const fvh_state_view *);
+                                        const fvh_state_view *, const double *,        \
+                                        const next_dt &);
 FVH_INSTANTIATE(2)
 FVH_INSTANTIATE(3)
 

@@ -1,0 +1,52 @@
+"""FP64 runs on both sides of every size at which the kernels change form (few
+cells or faces, one variable or two per thread), against the oracle bit for bit:
+a run of three steps carries dt from each corrector to the next step."""
+import numpy as np
+import pytest
+
+import flecsale_gb300.hydro as H
+from tests import _util as U
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dim,n,order", [
+    (2, (1, 1), 2), (2, (9, 7), 1), (2, (70, 70), 1),         # 9,940 faces
+    (2, (71, 70), 2),                                          # 10,081 faces
+    (2, (96, 64), 2), (2, (97, 64), 2),                        # 6,144 and 6,208 cells
+    (2, (160, 125), 2), (2, (160, 126), 1),                    # 20,000 and 20,160 cells
+    (3, (16, 16, 24), 2), (3, (17, 19, 20), 2),                # 6,144 and 6,460 cells
+    (3, (45, 32, 64), 2), (3, (46, 32, 64), 2),                # 92,160 and 94,208 cells
+    (2, (512, 512), 2), (2, (513, 512), 2)])                   # 262,144 and 262,656 cells
+def test_run_bitwise(cuda, oracle_lib, dim, n, order):
+    mesh = H.HostMesh.box(dim, n, [0] * dim, [1] * dim, 0.15, 5)
+    p = H.make_params(dim, flux="hllc" if dim == 2 else "rusanov", order=order, cfl=0.3,
+                      final_time=1e9)
+    x = mesh.arrays()["cell_centroid"]
+    w = 0.05 * np.sin(2 * np.pi * (2 * x + np.arange(dim)[:, None]))
+    state = H.state_from_dvp(dim, 1 + w.sum(0) + (x[0] < 0.5), w, 1 + 1.4 * w.sum(0) + (x[0] < 0.5))
+    one = state.copy()
+    st, t, _ = U.oracle_run(oracle_lib, mesh, state, p, 3)
+    dmesh, dstate = H.DeviceMesh(mesh), H.DeviceState(dim, mesh.num_cells)
+    solver = H.Solver(dmesh, p)
+    stream = cuda.cuda.Stream()
+    dstate.upload(one, stream)
+    solver.reset(0.0, stream)
+    if st != 0:  # (one cell has no neighbours: its least-squares system is singular)
+        with pytest.raises(H.FvhError) as e:
+            solver.run(dstate, 3, stream=stream)
+        assert e.value.code == st
+        return
+    assert solver.run(dstate, 3, stream=stream) == 3
+    out = dstate.download(stream)
+    stream.synchronize()
+    assert solver.soln_time(stream) == t and np.array_equal(out, state)
+    # step by step (each step takes dt from the state), then a run again
+    dstate.upload(one, stream)
+    solver.reset(0.0, stream)
+    for _ in range(2):
+        solver.step(dstate, stream)
+    solver.run(dstate, 1, stream=stream)
+    again = dstate.download(stream)
+    stream.synchronize()
+    assert np.array_equal(again, state)

@@ -22,6 +22,35 @@ __host__ __device__ inline unsigned long long status_key(long long cell, int cod
 }
 
 #ifdef __CUDACC__
+// Overlapped launches (programmatic dependent launch): a kernel launched with
+// overlap = true may start while its predecessor in the stream still runs.
+// Before `after_previous` it reads only what no kernel of a step writes (the
+// mesh, the tables); after it, everything the predecessors wrote is visible.
+// Every kernel of a step that may have such a successor calls it, so that a
+// kernel's end implies the end of all before it; `let_next_start` at a kernel's
+// start is what allows the overlap.  Launched without it both do nothing.
+__device__ __forceinline__ void let_next_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <class... P, class... A>
+inline cudaError_t launch(void (*kernel)(P...), dim3 grid, int threads, cudaStream_t st,
+                          bool overlap, const A &...args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = dim3(threads);
+  c.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // Block-wide maximum with the reference's std::max semantics; all threads of
 // the block must call it; the result is valid in thread 0.
 __device__ inline double block_max(double v) {
@@ -78,6 +107,8 @@ struct next_dt {
   fvh_device_status *status = nullptr;
 };
 
+// overlap (here and below): the kernel may start before its predecessor in the
+// stream has ended (see fvh::launch).
 template <int D>
 cudaError_t launch_dt(const fvh_mesh_view &m, const fvh_state_view &s,
                       const fvh_params &p, const double *soln_time, double *dt,
@@ -89,12 +120,12 @@ template <int D>
 cudaError_t launch_gradients(const fvh_mesh_view &m, const fvh_state_view &s,
                              const fvh_gradient_view &g, const fvh_params &p,
                              cudaStream_t st, const tables &t = tables(),
-                             const next_dt &nd = next_dt());
+                             const next_dt &nd = next_dt(), bool overlap = false);
 template <int D>
 cudaError_t launch_fluxes(const fvh_mesh_view &m, const fvh_state_view &s,
                           const fvh_gradient_view &g, const fvh_flux_view &fl,
                           const fvh_params &p, cudaStream_t st, const tables &t = tables(),
-                          const next_dt &nd = next_dt());
+                          const next_dt &nd = next_dt(), bool overlap = false);
 // Diagnostic: out[i] = a[i] op b[i] for op 0 mul, 1 add, 2 sub, 3 div on the
 // integer pipes (fvh_sf64.cuh), 4..7 the same with the FP64 instructions,
 // 8 / 9 the optimistic mul / div with their FP64 redo.
@@ -109,7 +140,8 @@ cudaError_t launch_update(const fvh_mesh_view &m, const fvh_params &p, const dou
                           const fvh_state_view &s, double *soln_time,
                           fvh_device_status *status, cudaStream_t st,
                           const fvh_state_view *out = nullptr,
-                          const double *slot_dx = nullptr, const next_dt &nd = next_dt());
+                          const double *slot_dx = nullptr, const next_dt &nd = next_dt(),
+                          bool overlap = false);
 }  // namespace plain
 
 }  // namespace fvh

@@ -140,10 +140,6 @@ struct arith_hw {
   __device__ __forceinline__ part take(double x) { return x; }
   __device__ __forceinline__ part take_entry(double x) { return x; }
   __device__ __forceinline__ double prod(part a, part b) { return __dmul_rn(a, b); }
-  __device__ __forceinline__ void add_first(double &s, part a, part b) {
-    s = 0.0 + __dmul_rn(a, b);
-  }
-  __device__ __forceinline__ void add(double &s, part a, part b) { s += __dmul_rn(a, b); }
   __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
   __device__ __forceinline__ double quo(double a, double b) { return __ddiv_rn(a, b); }
   __device__ __forceinline__ double half(double x) { return __dmul_rn(x, 0.5); }
@@ -690,7 +686,7 @@ __device__ __forceinline__ void vertex_offset(const fvh_mesh_view &m, const tabl
 // per-vertex minimum.
 template <int D, bool PRE>
 __device__ __noinline__ double limiter_exact(const fvh_mesh_view &m, const tables &t,
-                                             const double *__restrict__ plane, int c0, double u0,
+                                             const double *plane, int c0, double u0,
                                              double g0, double g1, double g2) {
   constexpr double tol = 1.e-9;
   const long long ktol = okey(tol), kntol = okey(-tol);
@@ -787,7 +783,7 @@ struct side_limit {
 // the integer pipes.  `rare` notes operands these leave to the hardware.
 template <int D, bool PRE, bool UP>
 __device__ __noinline__ side_limit limiter_side(const fvh_mesh_view &m, const tables &t,
-                                                const double *__restrict__ plane, int c0,
+                                                const double *plane, int c0,
                                                 double u0, double g0, double g1, double g2,
                                                 float E) {
   const double g[3] = {g0, g1, g2};
@@ -895,11 +891,11 @@ __device__ __forceinline__ void solve(A &ar, const double (&r)[10], const double
 // du <= tol, or du <= umax - u0 (RN(umax - u0) is the largest neighbour
 // difference, of which the key of the high half gives a lower bound), and
 // likewise below; phi is then 1 exactly.  The other variables take
-// limiter_exact.  In flows that are smooth or at rest up to rounding nearly
+// limiter_side.  In flows that are smooth or at rest up to rounding nearly
 // all are decided, which saves their vertex products and sums and the second
 // pass over the neighbours.
-template <int D, int NK, bool LIMIT, bool PRE, class A>
-__device__ __forceinline__ void cell_gradients(A &ar, const fvh_mesh_view &m,
+template <int D, int NK, bool LIMIT, bool PRE>
+__device__ __forceinline__ void cell_gradients(arith_opt &ar, const fvh_mesh_view &m,
                                                const fvh_state_view &s, const tables &t, int c0,
                                                int k0, const double (&r)[lsq_width<D>::value],
                                                double (&gu)[NK][D]) {
@@ -944,8 +940,8 @@ __device__ __forceinline__ void cell_gradients(A &ar, const fvh_mesh_view &m,
     }
     // a neighbour equal to the cell in every variable adds (+-0) * dx = +-0 to
     // each sum, which leaves it as it is: cells inside a uniform region skip it
-    if (A::wide_issue && same) return;
-    typename A::part px[D];
+    if (same) return;
+    sf64::parts px[D];
 #pragma unroll
     for (int j = 0; j < D; ++j) px[j] = PRE ? ar.take_entry(dx[j]) : ar.take(dx[j]);
 #pragma unroll
@@ -961,8 +957,7 @@ __device__ __forceinline__ void cell_gradients(A &ar, const fvh_mesh_view &m,
     }
   };
   if (q0 < q1) neighbour(q0, true);
-  constexpr int U = A::wide_issue ? 1 : 4;
-#pragma unroll U
+#pragma unroll 1
   for (int q = q0 + 1; q < q1; ++q) neighbour(q, false);
   {
     double lsq[lsq_width<D>::value];
@@ -985,7 +980,7 @@ __device__ __forceinline__ void cell_gradients(A &ar, const fvh_mesh_view &m,
     for (int i = 0; i < D; ++i) gf[k][i] = truncated(gu[k][i], wide[k]);
   }
   const int r0 = m.cell_vertex_offsets[c0], r1 = m.cell_vertex_offsets[c0 + 1];
-#pragma unroll U
+#pragma unroll 1
   for (int rr = r0; rr < r1; ++rr) {
     double dxv[D];
     float f[D];
@@ -1058,18 +1053,114 @@ __device__ __forceinline__ void store_gradients(const fvh_gradient_view &g, int 
     for (int i = 0; i < D; ++i) grad_planes_at<D>(g, k0 + k)[i][c0] = gu[k][i];
 }
 
-// the gradients of NK variables from k0 on of cell c0 with the FP64
-// instructions, stored
-template <int D, int NK, bool LIMIT, bool PRE>
-__device__ __forceinline__ void gradient_group_fp64(const fvh_mesh_view &m,
-                                                    const fvh_state_view &s,
-                                                    const fvh_gradient_view &g, const tables &t,
-                                                    int c0, int k0) {
-  double gu[NK][D], r[lsq_width<D>::value];
+// The limited gradient of variable k of cell c0 with the FP64 instructions,
+// stored: the reference's arithmetic in as short a chain as it has.  The vertex
+// offsets are read ahead, the neighbour extrema taken beside the sums, and every
+// vertex tested (limiter_exact says why the extreme differences suffice).
+// `ready` is called between reading the cell's lists and offsets and its state.
+template <int D, bool LIMIT, bool PRE, class READY>
+__device__ __forceinline__ void gradient_fp64(const fvh_mesh_view &m, const fvh_state_view &s,
+                                              const fvh_gradient_view &g, const tables &t, int c0,
+                                              int k, READY ready) {
   arith_hw hw;
+  const int q0 = m.cell_nbr_offsets[c0], q1 = m.cell_nbr_offsets[c0 + 1];
+  const int r0 = LIMIT ? m.cell_vertex_offsets[c0] : 0, r1 = LIMIT ? m.cell_vertex_offsets[c0 + 1] : 0;
+  double x0[D], r[lsq_width<D>::value];
+  if (!PRE) {
+#pragma unroll
+    for (int i = 0; i < D; ++i) x0[i] = m.cell_centroid[i][c0];
+  }
+  constexpr int AHEAD = D == 2 ? 4 : 8;
+  double ahead[AHEAD][D];
+  if (LIMIT) {
+#pragma unroll
+    for (int v = 0; v < AHEAD; ++v)
+      if (r0 + v < r1) vertex_offset<D, PRE>(m, t, r0 + v, x0, ahead[v]);
+  }
+  if (PRE) {
+#pragma unroll
+    for (int w = 0; w < lsq_width<D>::value; ++w) r[w] = t.lsq[(size_t)w * m.num_cells + c0];
+  }
+  constexpr int LISTED = 8;
+  int listed[LISTED];
+#pragma unroll
+  for (int i = 0; i < LISTED; ++i) listed[i] = q0 + i < q1 ? m.cell_nbrs[q0 + i] : 0;
+  ready();
+  const double *plane = state_plane_at<D>(s, k);
+  const double u0 = plane[c0];
+  double b[D];
+#pragma unroll
+  for (int j = 0; j < D; ++j) b[j] = 0;
+  long long kmin = okey(u0), kmax = kmin;
+  auto neighbour = [&](int q, int c1) {
+    const double u1 = plane[c1], du = u1 - u0;
+    double dx[D];
+    if (PRE) {
+      load_dx<D>(t.nbr_dx + (size_t)q * D, dx);
+    } else {
+#pragma unroll
+      for (int d = 0; d < D; ++d) dx[d] = m.cell_centroid[d][c1] - x0[d];
+    }
+#pragma unroll
+    for (int j = 0; j < D; ++j) b[j] += __dmul_rn(du, dx[j]);
+    if (LIMIT) {
+      const long long k1 = okey(u1);
+      kmin = (k1 < kmin) ? k1 : kmin;
+      kmax = (kmax < k1) ? k1 : kmax;
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < LISTED; ++i)
+    if (q0 + i < q1) neighbour(q0 + i, listed[i]);
+#pragma unroll 4
+  for (int q = q0 + LISTED; q < q1; ++q) neighbour(q, m.cell_nbrs[q]);
   if (!PRE) lsq_matrix<D>(hw, m, c0, r);
-  cell_gradients<D, NK, LIMIT, PRE>(hw, m, s, t, c0, k0, r, gu);
-  store_gradients<D, NK>(g, c0, k0, gu);
+  double gu[D];
+  solve(hw, r, b, gu);
+  if (LIMIT) {
+    constexpr double tol = 1.e-9;
+    const long long ktol = okey(tol), kntol = okey(-tol), one = okey(1.0);
+    long long kpos = 0, kneg = 0;
+    auto vertex = [&](const double *dxv) {
+      double u1 = u0;
+#pragma unroll
+      for (int i = 0; i < D; ++i) u1 += __dmul_rn(dxv[i], gu[i]);
+      const long long kd = okey(u1 - u0);
+      if (kd > ktol) kpos = (kpos < kd) ? kd : kpos;
+      else if (kd < kntol) kneg = (kd < kneg) ? kd : kneg;
+    };
+#pragma unroll
+    for (int v = 0; v < AHEAD; ++v)
+      if (r0 + v < r1) vertex(ahead[v]);
+#pragma unroll 1
+    for (int rr = r0 + AHEAD; rr < r1; ++rr) {
+      double dxv[D];
+      vertex_offset<D, PRE>(m, t, rr, x0, dxv);
+      vertex(dxv);
+    }
+    long long kphi = one;
+    if (kpos > ktol) {
+      const double num = from_okey(kmax) - u0;
+      if (okey(num) < kpos) {
+        const long long kq = okey(__ddiv_rn(num, from_okey(kpos)));
+        kphi = (kq < kphi) ? kq : kphi;
+      }
+    }
+    if (kneg < kntol) {
+      const double num = from_okey(kmin) - u0;
+      if (okey(num) > kneg) {
+        const long long kq = okey(__ddiv_rn(num, from_okey(kneg)));
+        kphi = (kq < kphi) ? kq : kphi;
+      }
+    }
+    kphi = (kphi < 0) ? 0 : kphi;  // std::max(phi, 0)
+    if (kphi != one) {
+#pragma unroll
+      for (int i = 0; i < D; ++i) gu[i] = __dmul_rn(gu[i], from_okey(kphi));
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < D; ++i) grad_planes_at<D>(g, k)[i][c0] = gu[i];
 }
 
 // the FP64 redo of a cell whose operands left the integer-pipe range, out of
@@ -1078,7 +1169,8 @@ template <int D, int NK, bool LIMIT, bool PRE>
 __device__ __noinline__ void gradient_group_hw(const fvh_mesh_view &m, const fvh_state_view &s,
                                                const fvh_gradient_view &g, const tables &t,
                                                int c0, int k0) {
-  gradient_group_fp64<D, NK, LIMIT, PRE>(m, s, g, t, c0, k0);
+#pragma unroll 1
+  for (int k = k0; k < k0 + NK; ++k) gradient_fp64<D, LIMIT, PRE>(m, s, g, t, c0, k, [] {});
 }
 
 // the gradients of NK variables from k0 on of cell c0, stored
@@ -1127,6 +1219,7 @@ __global__ void __launch_bounds__(kCellThreads, grad_min_blocks<D, PRE>())
 gradients_kernel(const __grid_constant__ fvh_mesh_view m, const __grid_constant__ fvh_state_view s,
                  const __grid_constant__ fvh_gradient_view g, const __grid_constant__ tables t,
                  const __grid_constant__ next_dt nd) {
+  after_previous();
   finish_dt(nd);
   const int c0 = blockIdx.x * blockDim.x + threadIdx.x;
   if (c0 >= m.num_cells) return;
@@ -1140,6 +1233,7 @@ gradients_kernel(const __grid_constant__ fvh_mesh_view m, const __grid_constant_
     gradient_group<D, G, LIMIT, PRE>(m, s, g, t, c0, k0, r, ar.rare);
   if constexpr (R != 0)
     if (k0 == NV - R) gradient_group<D, R, LIMIT, PRE>(m, s, g, t, c0, k0, r, ar.rare);
+  let_next_start();
 }
 
 // Few cells (kFewCells): one variable of one cell per thread (blockIdx.y), with
@@ -1150,10 +1244,13 @@ gradients_few_kernel(const __grid_constant__ fvh_mesh_view m,
                      const __grid_constant__ fvh_state_view s,
                      const __grid_constant__ fvh_gradient_view g,
                      const __grid_constant__ tables t, const __grid_constant__ next_dt nd) {
-  finish_dt(nd);
   const int c0 = blockIdx.x * blockDim.x + threadIdx.x;
   if (c0 >= m.num_cells) return;
-  gradient_group_fp64<D, 1, LIMIT, PRE>(m, s, g, t, c0, blockIdx.y);
+  gradient_fp64<D, LIMIT, PRE>(m, s, g, t, c0, blockIdx.y, [&] {
+    after_previous();
+    finish_dt(nd);
+  });
+  let_next_start();
 }
 
 // ---------------------------------------------------------------------------
@@ -1226,20 +1323,28 @@ __device__ __forceinline__ void face_offset(const fvh_mesh_view &m, const double
 }
 
 // the area-weighted flux of face f (tasks.h:405-461)
-template <int D, int KIND, bool SECOND, bool PRE, class A>
+struct at_once {
+  __device__ __forceinline__ void operator()() const {}
+};
+// `ready` is called between reading the face's geometry and its cells' state
+template <int D, int KIND, bool SECOND, bool PRE, class A, class READY = at_once>
 __device__ __forceinline__ void face_flux(A &ar, const fvh_mesh_view &m,
                                           const fvh_state_view &s, const fvh_gradient_view &g,
                                           int f, int2 cc, bool swap, bool outflow,
-                                          const double *face_dx, double *F) {
+                                          const double *face_dx, double *F,
+                                          READY ready = READY()) {
   double n[D];
 #pragma unroll
   for (int i = 0; i < D; ++i) n[i] = m.face_normal[i][f];
-  double dx[D] = {};
+  double dx[D] = {}, dx1[D] = {};
   if (SECOND) face_offset<D, PRE>(m, face_dx, f, 0, cc.x, dx);
+  // (many warps: the second offset is read where it is used)
+  if (SECOND && !A::wide_issue && cc.y >= 0) face_offset<D, PRE>(m, face_dx, f, 1, cc.y, dx1);
+  ready();
   const prim<D> wl = reconstruct<D, SECOND, PRE>(ar, s, g, cc.x, dx, swap);
   if (cc.y >= 0) {
-    if (SECOND) face_offset<D, PRE>(m, face_dx, f, 1, cc.y, dx);
-    const prim<D> wr = reconstruct<D, SECOND, PRE>(ar, s, g, cc.y, dx, swap);
+    if (SECOND && A::wide_issue) face_offset<D, PRE>(m, face_dx, f, 1, cc.y, dx1);
+    const prim<D> wr = reconstruct<D, SECOND, PRE>(ar, s, g, cc.y, dx1, swap);
     if (KIND == FVH_FLUX_RUSANOV)
       rusanov<D>(ar, wl, wr, n, F);
     else if (KIND == FVH_FLUX_HLLC)
@@ -1286,6 +1391,7 @@ fluxes_kernel(const __grid_constant__ fvh_mesh_view m, const __grid_constant__ f
               const __grid_constant__ fvh_gradient_view g, const __grid_constant__ fvh_flux_view fl,
               int swap, int outflow, const double *__restrict__ face_dx,
               const __grid_constant__ next_dt nd) {
+  after_previous();
   if (!SECOND) finish_dt(nd);  // (first order has no gradients)
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= m.num_faces) return;
@@ -1297,6 +1403,7 @@ fluxes_kernel(const __grid_constant__ fvh_mesh_view m, const __grid_constant__ f
     face_flux_hw<D, KIND, SECOND, PRE>(m, s, g, fl, f, cc, swap, outflow, face_dx);
     return;
   }
+  let_next_start();
   store_flux<D>(fl, f, F);
 }
 
@@ -1307,13 +1414,16 @@ fluxes_few_kernel(const __grid_constant__ fvh_mesh_view m, const __grid_constant
                   const __grid_constant__ fvh_gradient_view g,
                   const __grid_constant__ fvh_flux_view fl, int swap, int outflow,
                   const double *__restrict__ face_dx, const __grid_constant__ next_dt nd) {
-  if (!SECOND) finish_dt(nd);
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= m.num_faces) return;
   double F[D + 2];
   arith_hw hw;
   face_flux<D, KIND, SECOND, PRE>(hw, m, s, g, f, reinterpret_cast<const int2 *>(m.face_cells)[f],
-                                  swap != 0, outflow != 0, face_dx, F);
+                                  swap != 0, outflow != 0, face_dx, F, [&] {
+                                    after_previous();
+                                    if (!SECOND) finish_dt(nd);
+                                  });
+  let_next_start();
   store_flux<D>(fl, f, F);
 }
 
@@ -1330,47 +1440,59 @@ __device__ __forceinline__ double signed_flux(double F, bool minus) {
 // the new state of cell c: w = (d, v.., e, p, T, a^2)
 // gm1 = gamma - 1 and ggm1 = gamma * (gamma - 1), rounded once on the host
 // exactly as the reference rounds them per cell (euler_eqns.h / ideal_gas.h)
-template <int D, class A>
+// The lists are read before `ready` is called and the time increment
+// delta_t = dt * factor and the state after it.
+template <int D, class A, class READY = at_once>
 __device__ __forceinline__ void cell_update(A &ar, const fvh_mesh_view &m,
                                             const fvh_flux_view &fl, const fvh_state_view &s,
-                                            int c, double delta_t, double gm1, double ggm1,
-                                            double cv, double *w) {
+                                            int c, const double *dt, double factor, double gm1,
+                                            double ggm1, double cv, double *w,
+                                            READY ready = READY()) {
   double du[D + 2];
 #pragma unroll
   for (int k = 0; k < D + 2; ++k) du[k] = 0;
   const int q0 = m.cell_face_offsets[c], q1 = m.cell_face_offsets[c + 1];
-  constexpr int U = A::wide_issue ? 2 : 4;
-#pragma unroll U
-  for (int q = q0; q < q1; ++q) {
-    const int sf = m.cell_faces[q];
+  const double vol = m.cell_volume[c];
+  auto face = [&](int i, int sf) {
     const int f = sf < 0 ? ~sf : sf;
     double F[D + 2];
     F[0] = fl.mass[f];
 #pragma unroll
     for (int i = 0; i < D; ++i) F[1 + i] = fl.momentum[i][f];
     F[D + 1] = fl.energy[f];
-    // the first sum, 0 -+ F, is F with its sign
-    if (q == q0) {
+    if (i == 0) {  // the first sum, 0 -+ F, is F with its sign
 #pragma unroll
       for (int k = 0; k < D + 2; ++k) du[k] = signed_flux(F[k], sf >= 0);
-      continue;
-    }
-    // the update kernel's FP64 pipe is its bound: the next face's sums run on
-    // the integer pipe; a - b is a + (-b) exactly
-    if (A::wide_issue && q == q0 + 1) {
+    } else if (A::wide_issue && i == 1) {
+      // the update kernel's FP64 pipe is its bound: these sums run on the
+      // integer pipe; a - b is a + (-b) exactly
 #pragma unroll
       for (int k = 0; k < D + 2; ++k) du[k] = add_call(du[k], sf >= 0 ? -F[k] : F[k]);
-      continue;
-    }
-    if (sf >= 0) {
+    } else if (sf >= 0) {
 #pragma unroll
       for (int k = 0; k < D + 2; ++k) du[k] -= F[k];
     } else {
 #pragma unroll
       for (int k = 0; k < D + 2; ++k) du[k] += F[k];
     }
+  };
+  if (A::wide_issue) {
+    ready();
+#pragma unroll 2
+    for (int q = q0; q < q1; ++q) face(q - q0, m.cell_faces[q]);
+  } else {
+    constexpr int LISTED = 2 * D;
+    int listed[LISTED];
+#pragma unroll
+    for (int i = 0; i < LISTED; ++i) listed[i] = q0 + i < q1 ? m.cell_faces[q0 + i] : 0;
+    ready();
+#pragma unroll
+    for (int i = 0; i < LISTED; ++i)
+      if (q0 + i < q1) face(i, listed[i]);
+#pragma unroll 1
+    for (int q = q0 + LISTED; q < q1; ++q) face(q - q0, m.cell_faces[q]);
   }
-  const double scale = ar.quo(delta_t, m.cell_volume[c]);
+  const double scale = ar.quo(__dmul_rn(dt[0], factor), vol);
 #pragma unroll
   for (int k = 0; k < D + 2; ++k) du[k] = ar.mul(du[k], scale);
   double vel[D];
@@ -1402,19 +1524,19 @@ update_kernel(const __grid_constant__ fvh_mesh_view m, const __grid_constant__ f
               double ggm1, double cv, double *soln_time, fvh_device_status *status,
               const __grid_constant__ fvh_state_view out, int has_out,
               const double *__restrict__ slot_dx, const __grid_constant__ next_dt nd) {
-  const double delta_t = __dmul_rn(dt[0], factor);
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c == 0) soln_time[0] = 0.0 + soln_time[0] + delta_t;
   if (!NEXT && c >= m.num_cells) return;
   double dt_inv = 0;
   if (!NEXT || c < m.num_cells) {
     double w[D + 5];
     arith_opt ar;
-    if (!FEW) cell_update<D>(ar, m, fl, s, c, delta_t, gm1, ggm1, cv, w);
+    if (!FEW) cell_update<D>(ar, m, fl, s, c, dt, factor, gm1, ggm1, cv, w, after_previous);
     if (FEW || ar.rare) {
       arith_hw hw;
-      cell_update<D>(hw, m, fl, s, c, delta_t, gm1, ggm1, cv, w);
+      cell_update<D>(hw, m, fl, s, c, dt, factor, gm1, ggm1, cv, w, after_previous);
     }
+    if (c == 0) soln_time[0] = 0.0 + soln_time[0] + __dmul_rn(dt[0], factor);
+    let_next_start();
     const double a = sqrt(w[D + 4]);
     s.density[c] = w[0];
 #pragma unroll
@@ -1516,11 +1638,12 @@ cudaError_t launch_dt(const fvh_mesh_view &m, const fvh_state_view &s,
 template <int D>
 cudaError_t launch_gradients(const fvh_mesh_view &m, const fvh_state_view &s,
                              const fvh_gradient_view &g, const fvh_params &p,
-                             cudaStream_t st, const tables &t, const next_dt &nd) {
+                             cudaStream_t st, const tables &t, const next_dt &nd,
+                             bool overlap) {
   const bool lim = p.limiter != FVH_LIMITER_NONE, pre = t.lsq && t.nbr_dx && t.vtx_dx;
   if (m.num_cells <= (pre ? kFewCells : kFewCellsNoTables)) {
     const dim3 grid(blocks_of(m.num_cells, kFewThreads), D + 4);
-    auto go = [&](auto kernel) { kernel<<<grid, kFewThreads, 0, st>>>(m, s, g, t, nd); };
+    auto go = [&](auto kernel) { launch(kernel, grid, kFewThreads, st, overlap, m, s, g, t, nd); };
     if (pre)
       lim ? go(gradients_few_kernel<D, true, true>) : go(gradients_few_kernel<D, false, true>);
     else
@@ -1529,7 +1652,7 @@ cudaError_t launch_gradients(const fvh_mesh_view &m, const fvh_state_view &s,
   }
   auto go = [&](auto kernel, int groups) {
     const dim3 grid(blocks_of(m.num_cells, kCellThreads), groups);
-    kernel<<<grid, kCellThreads, 0, st>>>(m, s, g, t, nd);
+    launch(kernel, grid, kCellThreads, st, overlap, m, s, g, t, nd);
   };
   const int pairs = blocks_of(D + 4, 2);
   if (!pre)
@@ -1585,10 +1708,10 @@ template <int D, bool SECOND, bool PRE>
 static void launch_fluxes_kind(const fvh_mesh_view &m, const fvh_state_view &s,
                                const fvh_gradient_view &g, const fvh_flux_view &fl,
                                const fvh_params &p, cudaStream_t st, const double *face_dx,
-                               const next_dt &nd) {
+                               const next_dt &nd, bool overlap) {
   auto go = [&](auto kernel, int threads) {
-    kernel<<<blocks_of(m.num_faces, threads), threads, 0, st>>>(m, s, g, fl, p.recon_swap_ep,
-                                                               p.boundary, face_dx, nd);
+    launch(kernel, blocks_of(m.num_faces, threads), threads, st, overlap, m, s, g, fl,
+           p.recon_swap_ep, p.boundary, face_dx, nd);
   };
   auto kind = [&](auto k) {
     constexpr int KIND = decltype(k)::value;
@@ -1609,13 +1732,13 @@ template <int D>
 cudaError_t launch_fluxes(const fvh_mesh_view &m, const fvh_state_view &s,
                           const fvh_gradient_view &g, const fvh_flux_view &fl,
                           const fvh_params &p, cudaStream_t st, const tables &t,
-                          const next_dt &nd) {
+                          const next_dt &nd, bool overlap) {
   if (p.order == 1)
-    launch_fluxes_kind<D, false, false>(m, s, g, fl, p, st, nullptr, nd);
+    launch_fluxes_kind<D, false, false>(m, s, g, fl, p, st, nullptr, nd, overlap);
   else if (t.face_dx)
-    launch_fluxes_kind<D, true, true>(m, s, g, fl, p, st, t.face_dx, nd);
+    launch_fluxes_kind<D, true, true>(m, s, g, fl, p, st, t.face_dx, nd, overlap);
   else
-    launch_fluxes_kind<D, true, false>(m, s, g, fl, p, st, nullptr, nd);
+    launch_fluxes_kind<D, true, false>(m, s, g, fl, p, st, nullptr, nd, overlap);
   return cudaGetLastError();
 }
 
@@ -1624,15 +1747,15 @@ cudaError_t launch_update(const fvh_mesh_view &m, const fvh_params &p, const dou
                           double factor, const fvh_flux_view &fl,
                           const fvh_state_view &s, double *soln_time,
                           fvh_device_status *status, cudaStream_t st,
-                          const fvh_state_view *out, const double *slot_dx, const next_dt &nd) {
+                          const fvh_state_view *out, const double *slot_dx, const next_dt &nd,
+                          bool overlap) {
   // the same two roundings as (gamma - 1.0) and gamma * (gamma - 1.0) per cell
   const double gamma = p.gamma;
   const double gm1 = gamma - 1.0;
   const double ggm1 = gamma * gm1;
   auto go = [&](auto kernel, int threads) {
-    kernel<<<blocks_of(m.num_cells, threads), threads, 0, st>>>(
-        m, fl, s, dt, factor, gm1, ggm1, p.cv, soln_time, status, out ? *out : s, out ? 1 : 0,
-        slot_dx, nd);
+    launch(kernel, blocks_of(m.num_cells, threads), threads, st, overlap, m, fl, s, dt, factor, gm1,
+           ggm1, p.cv, soln_time, status, out ? *out : s, out ? 1 : 0, slot_dx, nd);
   };
   if (m.num_cells <= kFewUpdateCells)
     nd.maximum ? go(update_kernel<D, true, true>, kFewThreads)
@@ -1651,19 +1774,19 @@ cudaError_t launch_update(const fvh_mesh_view &m, const fvh_params &p, const dou
                                     unsigned long long *);                             \
   template cudaError_t launch_gradients<D>(const fvh_mesh_view &, const fvh_state_view &, \
                                            const fvh_gradient_view &, const fvh_params &, \
-                                           cudaStream_t, const tables &, const next_dt &);              \
+                                           cudaStream_t, const tables &, const next_dt &, bool);              \
   template cudaError_t build_tables<D>(const fvh_mesh_view &, double *, int64_t, int64_t, \
                                        int64_t, tables *);                             \
   template cudaError_t launch_fluxes<D>(const fvh_mesh_view &, const fvh_state_view &, \
                                         const fvh_gradient_view &, const fvh_flux_view &, \
                                         const fvh_params &, cudaStream_t, const tables &, \
-                                        const next_dt &); \
+                                        const next_dt &, bool); \
   template cudaError_t launch_update<D>(const fvh_mesh_view &, const fvh_params &,     \
                                         const double *, double, const fvh_flux_view &, \
                                         const fvh_state_view &, double *,              \
                                         fvh_device_status *, cudaStream_t,             \
                                         const fvh_state_view *, const double *,        \
-                                        const next_dt &);
+                                        const next_dt &, bool);
 FVH_INSTANTIATE(2)
 FVH_INSTANTIATE(3)
 

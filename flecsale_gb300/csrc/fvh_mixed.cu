@@ -50,17 +50,25 @@ using phys::smin;
 
 constexpr int kMaxColours = 32;
 
-// per-cell AoS record sizes in float4 units
+// per-cell and per-face record sizes in float4 units.
+//
+// A record of more than 32 bytes is kept in planes of at most 32 bytes: a warp's
+// lanes hold consecutive cells or faces nearly always, so a plane is read and
+// written in full 128-byte lines, while one load of every 96th byte touches a
+// line for nearly every lane.  With whole records the 3D face fluxes spent 77 %
+// of the L1's line accesses on this (128^3: 177 -> 160 us, gradients 267 -> 260,
+// updates 128 -> 120).
+// 32 bytes is also one sector, so a lone cell's record costs no more.
 template <int D>
 struct layout {
   static constexpr int NV = D + 4;             // d, v[D], e, p, a
   static constexpr int PACK4 = 2;              // d v.. p e a (8 floats)
-  static constexpr int GRAD4 = D == 2 ? 3 : 6; // NV*D floats, padded
+  static constexpr int GRAD4 = D == 2 ? 3 : 6; // NV*D floats, padded (planes 2+1 or 2+2+2)
   static constexpr int CEN4 = D == 2 ? 1 : 2;  // centroid hi/lo
+  static constexpr int LSQ4 = D == 2 ? 0 : 2;  // sum of dx dx^T
   static constexpr int FGEO4 = 1;              // normal[D], area
   static constexpr int FDX4 = D == 2 ? 1 : 2;  // x_f - x_c0, x_f - x_c1
-  static constexpr int FLUX4 = D == 2 ? 1 : 2; // face flux (D+2 floats, padded)
-  static constexpr int DEL4 = D == 2 ? 2 : 3;  // predictor increments (D+2 double-floats)
+  static constexpr int DEL4 = D == 2 ? 2 : 3;  // predictor increments, D+2 double-floats (2+1)
 };
 
 // Staged 2D gradients (gradients_staged_kernel).  A chunk is a set of up to
@@ -71,6 +79,18 @@ struct stage_run {
   int first, count, slot, kind;
 };
 
+// What is copied for a chunk, in 16-byte slots: the head, then one run a slot.
+struct stage_head {
+  int runs;                // how many
+  unsigned bytes;          // all bytes the chunk's copies bring
+  unsigned topo_at;        // its topology block: place in stage_tables::topo and size, in
+  unsigned topo_units;     // 16-byte units
+};
+union stage_list {
+  stage_head head;
+  stage_run run;
+};
+
 struct stage_tables {
   int nchunks = 0;
   // layout of one stage buffer (bytes), sized for this mesh's largest chunk:
@@ -78,10 +98,8 @@ struct stage_tables {
   // (16 B) at vtx_at, the chunk's topology block at topo_at
   int cen_at = 0, vtx_at = 0, topo_at = 0, stage_bytes = 0;
   const int *cells = nullptr;                // [nchunks * kStageCells] cell ids, -1 = none
-  const int *run_off = nullptr;              // [nchunks + 1] into runs
-  const stage_run *runs = nullptr;
-  const long long *topo_off = nullptr;       // [nchunks + 1] byte offsets into topo
-  const unsigned *bytes = nullptr;           // [nchunks] bytes staged per chunk
+  const stage_list *lists = nullptr;         // [nchunks * list_slots]: a head, then the runs
+  int list_slots = 0;                        // slots of a chunk's list
   const unsigned *topo = nullptr;            // per chunk: see setup_stage_host
 };
 
@@ -93,9 +111,11 @@ struct workspace {
   float4 *grads = nullptr;
   float4 *ccen = nullptr;    // cell centroid hi/lo
   float4 *vcoord = nullptr;  // vertex coordinates hi/lo
+  float4 *lsq = nullptr;     // 3D: least-squares sums of dx dx^T (6 floats of 8)
   float4 *fgeo = nullptr;    // face normal + area
   float4 *fdx = nullptr;     // face centroid offsets from both cells
-  float4 *fflux = nullptr;   // face schedule: area-scaled face fluxes
+  float4 *fflux = nullptr;   // face schedule: area-scaled face fluxes, the first four
+  float *fflux5 = nullptr;   // 3D: the fifth (energy)
   float4 *delta = nullptr;   // predictor increments of (d, v.., e) as double-floats
   float *inv_vol32 = nullptr;  // 1/V rounded to FP32 (CFL estimate; update, high part)
   float *inv_vol_lo = nullptr; // 1/V - inv_vol32, rounded to FP32 (update, low part)
@@ -155,33 +175,62 @@ __device__ __forceinline__ prim<float, D> load_pack(const float4 *pk, int c) {
 template <int D>
 __device__ __forceinline__ void store_pack(float4 *pk, int c, float d, const float *v, float p,
                                            float e, float a) {
-  if (D == 2) {
-    pk[2 * (size_t)c] = make_float4(d, v[0], v[1], p);
-    pk[2 * (size_t)c + 1] = make_float4(e, a, 0.f, 0.f);
-  } else {
-    pk[2 * (size_t)c] = make_float4(d, v[0], v[1], v[D - 1]);
-    pk[2 * (size_t)c + 1] = make_float4(p, e, a, 0.f);
-  }
+  if (D == 2)
+    stg256(pk + 2 * (size_t)c, make_float4(d, v[0], v[1], p), make_float4(e, a, 0.f, 0.f));
+  else
+    stg256(pk + 2 * (size_t)c, make_float4(d, v[0], v[1], v[D - 1]), make_float4(p, e, a, 0.f));
 }
 
-// gradient record: g[k*D + i] = d u_k / d x_i, u = (d, v.., e, p, a)
-template <int D>
-__device__ __forceinline__ void load_grads(const float4 *gr, int c, float *g) {
-  constexpr int G4 = layout<D>::GRAD4;
-  float4 t[G4];
-  if (G4 % 2 == 0) {  // 32-byte aligned records: 256-bit loads
+// Records in planes: N4 float4 of record c out of n, two to a plane (the last
+// plane holds one when N4 is odd).
+template <int N4>
+__device__ __forceinline__ void load_planes(const float4 *base, int n, int c, float *x) {
+  float4 t[N4];
 #pragma unroll
-    for (int q = 0; q < G4; q += 2) ldg256(gr + (size_t)G4 * c + q, t[q], t[q + 1]);
+  for (int q = 0; q + 1 < N4; q += 2) ldg256(base + (size_t)q * n + 2 * (size_t)c, t[q], t[q + 1]);
+  if (N4 % 2) t[N4 - 1] = base[(size_t)(N4 - 1) * n + c];
+#pragma unroll
+  for (int q = 0; q < N4; ++q) {
+    x[4 * q] = t[q].x;
+    x[4 * q + 1] = t[q].y;
+    x[4 * q + 2] = t[q].z;
+    x[4 * q + 3] = t[q].w;
+  }
+}
+// 2D gradients (48 bytes) stay whole records: the staged kernel takes its cells
+// in Morton order, where the two planes cost it more (51.5 -> 54.7 us at 1024^2)
+// than they save the face fluxes (40.4 -> 39.5).
+template <int D>
+__device__ __forceinline__ void load_grads(const float4 *gr, int n, int c, float *g) {
+  if constexpr (D == 3) {
+    load_planes<layout<D>::GRAD4>(gr, n, c, g);
   } else {
 #pragma unroll
-    for (int q = 0; q < G4; ++q) t[q] = gr[(size_t)G4 * c + q];
+    for (int q = 0; q < 3; ++q) {
+      const float4 t = gr[3 * (size_t)c + q];
+      g[4 * q] = t.x;
+      g[4 * q + 1] = t.y;
+      g[4 * q + 2] = t.z;
+      g[4 * q + 3] = t.w;
+    }
   }
+}
+template <int N4>
+__device__ __forceinline__ void store_planes(float4 *base, int n, int c, const float *x) {
+  auto at = [&](int q) { return make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]); };
 #pragma unroll
-  for (int q = 0; q < G4; ++q) {
-    g[4 * q] = t[q].x;
-    g[4 * q + 1] = t[q].y;
-    g[4 * q + 2] = t[q].z;
-    g[4 * q + 3] = t[q].w;
+  for (int q = 0; q + 1 < N4; q += 2) stg256(base + (size_t)q * n + 2 * (size_t)c, at(q), at(q + 1));
+  if (N4 % 2) base[(size_t)(N4 - 1) * n + c] = at(N4 - 1);
+}
+
+template <int D>
+__device__ __forceinline__ void store_grads(float4 *gr, int n, int c, const float *g) {
+  if constexpr (D == 3) {
+    store_planes<layout<D>::GRAD4>(gr, n, c, g);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      gr[3 * (size_t)c + q] = make_float4(g[4 * q], g[4 * q + 1], g[4 * q + 2], g[4 * q + 3]);
   }
 }
 
@@ -329,6 +378,30 @@ __global__ void setup_cells(const fvh_mesh_view m, workspace w) {
   w.inv_vol_lo[c] = iv.y;
 }
 
+// 3D: the sums of dx dx^T over the neighbours, formed once per mesh in the order
+// and precision of the gradients' loop (six of its 26 x 65 operations a cell and
+// six live registers; gradients 260 -> 256 us at 128^3)
+__global__ void setup_lsq(const fvh_mesh_view m, workspace w) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= m.num_cells) return;
+  float xh[3], xl[3], M[6] = {0, 0, 0, 0, 0, 0};
+  load_cen<3>(w.ccen, c, xh, xl);
+  for (int q = m.cell_nbr_offsets[c]; q < m.cell_nbr_offsets[c + 1]; ++q) {
+    float yh[3], yl[3], dx[3];
+    load_cen<3>(w.ccen, m.cell_nbrs[q], yh, yl);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) dx[i] = (yh[i] - xh[i]) + (yl[i] - xl[i]);
+    M[0] += dx[0] * dx[0];
+    M[1] += dx[0] * dx[1];
+    M[2] += dx[0] * dx[2];
+    M[3] += dx[1] * dx[1];
+    M[4] += dx[1] * dx[2];
+    M[5] += dx[2] * dx[2];
+  }
+  stg256(w.lsq + 2 * (size_t)c, make_float4(M[0], M[1], M[2], M[3]),
+         make_float4(M[4], M[5], 0.f, 0.f));
+}
+
 template <int D>
 __global__ void setup_vertices(const fvh_mesh_view m, workspace w) {
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
@@ -372,9 +445,9 @@ __global__ void setup_faces(const fvh_mesh_view m, workspace w) {
   }
 }
 
-template <int D>
+template <int D, bool STREAM = false>
 __device__ __forceinline__ void face_geo(const workspace &w, int f, float *n, float &area) {
-  const float4 g = w.fgeo[f];
+  const float4 g = STREAM ? __ldcs(w.fgeo + f) : w.fgeo[f];
   n[0] = g.x;
   n[1] = g.y;
   if (D == 2) {
@@ -587,13 +660,12 @@ __device__ __forceinline__ void pack_values(const prim<float, D> &p, float *u) {
   u[k++] = p.a;
 }
 
-template <int D, bool LIMIT, int UNROLL, class NBR>
-__device__ __forceinline__ void cell_gradients(const fvh_mesh_view &m, const workspace &w,
-                                               int c0, const float *u0, const float *xh,
-                                               const float *xl, int nn, NBR nbr) {
+template <int D, bool LIMIT, int UNROLL, class NBR, class VTX>
+__device__ __forceinline__ void cell_gradients(const workspace &w, int c0, const float *u0,
+                                               const float *xh, const float *xl, int nn, NBR nbr,
+                                               int nr, VTX vtx) {
   constexpr int NV = D + 4;
   constexpr float tol = 1.e-9f;
-  float M[6] = {0, 0, 0, 0, 0, 0};
   float b[NV][D];
   // neighbour extrema (tasks.h:232-236), taken in the same pass
   float umin[NV], umax[NV];
@@ -609,18 +681,6 @@ __device__ __forceinline__ void cell_gradients(const fvh_mesh_view &m, const wor
     nbr(q, u1, yh, yl);
 #pragma unroll
     for (int i = 0; i < D; ++i) dx[i] = (yh[i] - xh[i]) + (yl[i] - xl[i]);
-    if (D == 2) {
-      M[0] += dx[0] * dx[0];
-      M[1] += dx[0] * dx[1];
-      M[2] += dx[1] * dx[1];
-    } else {
-      M[0] += dx[0] * dx[0];
-      M[1] += dx[0] * dx[1];
-      M[2] += dx[0] * dx[D - 1];
-      M[3] += dx[1] * dx[1];
-      M[4] += dx[1] * dx[D - 1];
-      M[5] += dx[D - 1] * dx[D - 1];
-    }
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
       const float du = u1[k] - u0[k];
@@ -631,16 +691,10 @@ __device__ __forceinline__ void cell_gradients(const fvh_mesh_view &m, const wor
     }
   }
   float g[NV][D];
-  if (D == 2) {
-    const float det = M[0] * M[2] - M[1] * M[1];
-    const float inv = 1.f / det;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      g[k][0] = (b[k][0] * M[2] - b[k][1] * M[1]) * inv;
-      g[k][1] = (b[k][1] * M[0] - b[k][0] * M[1]) * inv;
-    }
-  } else {
-    const float a00 = M[0], a01 = M[1], a02 = M[2], a11 = M[3], a12 = M[4], a22 = M[5];
+  {
+    float4 m0, m1;
+    ldg256(w.lsq + 2 * (size_t)c0, m0, m1);
+    const float a00 = m0.x, a01 = m0.y, a02 = m0.z, a11 = m0.w, a12 = m1.x, a22 = m1.y;
     const float c00 = a11 * a22 - a12 * a12;
     const float c01 = a02 * a12 - a01 * a22;
     const float c02 = a01 * a12 - a02 * a11;
@@ -660,7 +714,6 @@ __device__ __forceinline__ void cell_gradients(const fvh_mesh_view &m, const wor
     float dpos[NV], dneg[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) dpos[k] = dneg[k] = 0.f;
-    const int r0 = m.cell_vertex_offsets[c0], nr = m.cell_vertex_offsets[c0 + 1] - r0;
     auto vertex = [&](const float *dxv) {
 #pragma unroll
       for (int k = 0; k < NV; ++k) {
@@ -673,7 +726,7 @@ __device__ __forceinline__ void cell_gradients(const fvh_mesh_view &m, const wor
     };
     for (int r = 0; r < nr; ++r) {
       float vh[3], vl[3], dxv[3];
-      load_cen<D>(w.vcoord, m.cell_vertices[r0 + r], vh, vl);
+      vtx(r, vh, vl);
 #pragma unroll
       for (int i = 0; i < D; ++i) dxv[i] = __fadd_rn(__fsub_rn(vh[i], xh[i]), __fsub_rn(vl[i], xl[i]));
       vertex(dxv);
@@ -696,10 +749,8 @@ __device__ __forceinline__ void cell_gradients(const fvh_mesh_view &m, const wor
     for (int i = 0; i < D; ++i) flat[k * D + i] = g[k][i];
 #pragma unroll
   for (int q = NV * D; q < 4 * G4; ++q) flat[q] = 0.f;
-#pragma unroll
-  for (int q = 0; q < G4; ++q)
-    w.grads[(size_t)G4 * c0 + q] =
-        make_float4(flat[4 * q], flat[4 * q + 1], flat[4 * q + 2], flat[4 * q + 3]);
+  // gradient record: flat[k*D + i] = d u_k / d x_i, u = (d, v.., e, p, a)
+  store_grads<D>(w.grads, w.nc, c0, flat);
 }
 
 // Packed FP32 pairs (the FADD2/FMUL2/FFMA2 instructions of sm_100+): each lane
@@ -889,10 +940,8 @@ __device__ __forceinline__ void cell_gradients_pairs(const workspace &w, int c0,
   }
 #pragma unroll
   for (int q = NV * D; q < 4 * G4; ++q) flat[q] = 0.f;
-#pragma unroll
-  for (int q = 0; q < G4; ++q)
-    w.grads[(size_t)G4 * c0 + q] =
-        make_float4(flat[4 * q], flat[4 * q + 1], flat[4 * q + 2], flat[4 * q + 3]);
+  // gradient record: flat[k*D + i] = d u_k / d x_i, u = (d, v.., e, p, a)
+  store_grads<D>(w.grads, w.nc, c0, flat);
 }
 
 // Neighbour records are loaded as the loop reaches them.  3D keeps
@@ -907,10 +956,13 @@ gradients_kernel(const fvh_mesh_view m, workspace w, const float4 *__restrict__ 
     float xh[3], xl[3];
     load_cen<D>(w.ccen, c0, xh, xl);
     const int q0 = m.cell_nbr_offsets[c0], nn = m.cell_nbr_offsets[c0 + 1] - q0;
+    const int r0 = m.cell_vertex_offsets[c0], nr = m.cell_vertex_offsets[c0 + 1] - r0;
+    auto vtx = [&](int r, float *vh, float *vl) {
+      load_cen<D>(w.vcoord, m.cell_vertices[r0 + r], vh, vl);
+    };
     if (D == 2) {
       float4 a0, b0;
       ldg256(pk + 2 * (size_t)c0, a0, b0);
-      const int r0 = m.cell_vertex_offsets[c0], nr = m.cell_vertex_offsets[c0 + 1] - r0;
       cell_gradients_pairs<D, LIMIT, 4>(
           w, c0, a0, b0, xh, xl, nn,
           [&](int q, float4 &a, float4 &b, float *yh, float *yl) {
@@ -918,16 +970,18 @@ gradients_kernel(const fvh_mesh_view m, workspace w, const float4 *__restrict__ 
             ldg256(pk + 2 * (size_t)c1, a, b);
             load_cen<D>(w.ccen, c1, yh, yl);
           },
-          nr, [&](int r, float *vh, float *vl) { load_cen<D>(w.vcoord, m.cell_vertices[r0 + r], vh, vl); });
+          nr, vtx);
     } else {
       float u0[D + 4];
       pack_values<D>(load_pack<D>(pk, c0), u0);
-      cell_gradients<D, LIMIT, 4>(m, w, c0, u0, xh, xl, nn,
-                                  [&](int q, float *u1, float *yh, float *yl) {
-                                    const int c1 = m.cell_nbrs[q0 + q];
-                                    pack_values<D>(load_pack<D>(pk, c1), u1);
-                                    load_cen<D>(w.ccen, c1, yh, yl);
-                                  });
+      cell_gradients<D, LIMIT, 4>(
+          w, c0, u0, xh, xl, nn,
+          [&](int q, float *u1, float *yh, float *yl) {
+            const int c1 = m.cell_nbrs[q0 + q];
+            pack_values<D>(load_pack<D>(pk, c1), u1);
+            load_cen<D>(w.ccen, c1, yh, yl);
+          },
+          nr, vtx);
     }
   }
 }
@@ -958,30 +1012,41 @@ constexpr int kStageMaxBytes = 24576; // one stage buffer at most (two per block
 constexpr int kStageWaitPolls = 1 << 22;  // bounded waits on a chunk's copies
 
 template <bool LIMIT>
-__global__ void __launch_bounds__(kStageCells)
+__global__ void __launch_bounds__(kStageCells, 7)
 gradients_staged_kernel(const fvh_mesh_view m, workspace w, const float4 *__restrict__ pk,
                         stage_tables t, int rev, fvh_device_status *status) {
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(8) unsigned long long bar[2];
+  __shared__ __align__(8) unsigned long long bar[2], list_bar[2];
+  stage_list *lists = reinterpret_cast<stage_list *>(smem + 2 * (size_t)t.stage_bytes);
   const int tid = threadIdx.x;
   auto chunk_at = [&](int i) { return rev ? t.nchunks - 1 - i : i; };
-  // posts the copies of chunk k into stage buffer b (warp 0)
-  auto post = [&](int k, int b) {
-    const int r0 = t.run_off[k], nr = t.run_off[k + 1] - r0;
-    const long long tb0 = t.topo_off[k];
-    const unsigned topo_bytes = (unsigned)(t.topo_off[k + 1] - tb0);
+  // A chunk's list is copied one chunk before it is posted, so that posting waits
+  // for no load: when warp 0 read the lists from memory at the post, it came to
+  // each chunk's barrier three dependent loads after the others (1024^2: 51.6 ->
+  // 49.0 us a launch; with the lists in registers, 96 of them, 54.8).
+  auto fetch_list = [&](int k, int b) {
+    if (tid != 0) return;
+    const unsigned bytes = (unsigned)t.list_slots * 16u;
+    tma::mbar_arrive_expect_tx(&list_bar[b], bytes);
+    tma::bulk_g2s(lists + b * t.list_slots, t.lists + (size_t)k * t.list_slots, bytes, &list_bar[b]);
+  };
+  // posts the copies of the chunk whose list is in list buffer b into stage
+  // buffer b (warp 0)
+  auto post = [&](int b) {
+    const stage_list *l = lists + b * t.list_slots;
+    const stage_head h = l->head;
     unsigned char *base = smem + (size_t)b * t.stage_bytes;
     // this buffer's earlier reads (ordered by the block barrier) come before
     // the copies that overwrite it
     tma::fence_proxy_async_shared();
     if (tid == 0) {
-      tma::mbar_arrive_expect_tx(&bar[b], t.bytes[k]);
-      tma::bulk_g2s(base + t.topo_at, reinterpret_cast<const unsigned char *>(t.topo) + tb0,
-                    topo_bytes, &bar[b]);
+      tma::mbar_arrive_expect_tx(&bar[b], h.bytes);
+      tma::bulk_g2s(base + t.topo_at, reinterpret_cast<const uint4 *>(t.topo) + h.topo_at,
+                    h.topo_units * 16u, &bar[b]);
     }
     __syncwarp();
-    for (int r = tid; r < nr; r += 32) {
-      const stage_run run = t.runs[r0 + r];
+    for (int r = tid; r < h.runs; r += 32) {
+      const stage_run run = l[1 + r].run;
       if (run.kind == 0) {
         tma::bulk_g2s(base + (size_t)run.slot * 32, pk + 2 * (size_t)run.first,
                       (unsigned)run.count * 32u, &bar[b]);
@@ -996,29 +1061,52 @@ gradients_staged_kernel(const fvh_mesh_view m, workspace w, const float4 *__rest
   if (tid == 0) {
     tma::mbar_init(&bar[0], 1);
     tma::mbar_init(&bar[1], 1);
+    tma::mbar_init(&list_bar[0], 1);
+    tma::mbar_init(&list_bar[1], 1);
     tma::fence_barrier_init();
   }
   __syncthreads();
-  // copies posted into / phases consumed from each buffer (the same in every
-  // thread: the decisions below are uniform across the block)
-  int posted[2] = {0, 0}, used[2] = {0, 0};
-  if ((int)blockIdx.x < t.nchunks) {
-    if (tid < 32) post(chunk_at(blockIdx.x), 0);
-    posted[0] = 1;
-  }
-  int it = 0;
-  for (int i = blockIdx.x; i < t.nchunks; i += gridDim.x, ++it) {
-    const int b = it & 1;
-    // the other buffer was last read by the previous chunk, before the
-    // barrier that ended it
-    if (i + (int)gridDim.x < t.nchunks) {
-      if (tid < 32) post(chunk_at(i + gridDim.x), b ^ 1);
-      ++posted[b ^ 1];
+  // Chunk `it` of this block uses the buffers it & 1, whose barriers then are in
+  // phase (it >> 1) & 1.  Its list is fetched during chunk it - 2, its copies
+  // are posted at the start of chunk it - 1.
+  const int step = gridDim.x;
+  const int mine = (int)blockIdx.x < t.nchunks ? (t.nchunks - 1 - (int)blockIdx.x) / step + 1 : 0;
+  auto chunk_of = [&](int it) { return chunk_at((int)blockIdx.x + it * step); };
+  bool landed = true;
+  if (mine > 0) {
+    fetch_list(chunk_of(0), 0);
+    if (mine > 1) fetch_list(chunk_of(1), 1);
+    if (tid < 32) {
+      landed = __all_sync(0xffffffffu, tma::mbar_wait_bounded(&list_bar[0], 0u, kStageWaitPolls));
+      if (landed) post(0);
     }
-    const int k = chunk_at(i);
-    const int c0 = t.cells[(size_t)k * kStageCells + tid];
-    const bool landed = tma::mbar_wait_bounded(&bar[b], (unsigned)(used[b] & 1), kStageWaitPolls);
-    ++used[b];
+  }
+  int c_ahead = mine > 0 ? t.cells[(size_t)chunk_of(0) * kStageCells + tid] : -1;
+  int listed = mine < 2 ? mine : 2, posted = 1;  // chunks whose list is fetched / copies are posted
+  for (int it = 0; it < mine; ++it) {
+    const int b = it & 1;
+    const unsigned phase = (unsigned)(it >> 1) & 1u;
+    const int k = chunk_of(it);
+    const int c0 = c_ahead;
+    // buffers b ^ 1 were last read during the previous chunk (lists: at its
+    // start), before the barrier that ended it
+    if (it + 1 < mine) {
+      if (tid < 32 && landed) {
+        landed = __all_sync(0xffffffffu,
+                            tma::mbar_wait_bounded(&list_bar[b ^ 1], (unsigned)((it + 1) >> 1) & 1u,
+                                                   kStageWaitPolls));
+        if (landed) post(b ^ 1);
+      }
+      ++posted;
+      c_ahead = t.cells[(size_t)chunk_of(it + 1) * kStageCells + tid];
+    }
+    // list buffer b was read when this chunk was posted, a barrier ago
+    if (it + 2 < mine) {
+      tma::fence_proxy_async_shared();
+      fetch_list(chunk_of(it + 2), b);
+      ++listed;
+    }
+    if (landed) landed = tma::mbar_wait_bounded(&bar[b], phase, kStageWaitPolls);
     const unsigned char *base = smem + (size_t)b * t.stage_bytes;
     const float4 *spk = reinterpret_cast<const float4 *>(base);
     const float4 *scen = reinterpret_cast<const float4 *>(base + t.cen_at);
@@ -1054,12 +1142,14 @@ gradients_staged_kernel(const fvh_mesh_view m, workspace w, const float4 *__rest
     // buffer before it is posted again, and a wait that ran out anywhere
     // stops the whole block
     if (__syncthreads_or(!landed)) {
-      // report, then wait (bounded) for every posted copy before leaving, so
+      // report, then wait (bounded) for every copy under way before leaving, so
       // none lands in shared memory this block no longer owns
       if (tid == 0) atomicMin(status, status_key(t.cells[(size_t)k * kStageCells], FVH_ERR_TIMEOUT));
-      for (int bb = 0; bb < 2; ++bb)  // (a phase that completed returns at once)
-        if (posted[bb] > 0)
-          tma::mbar_wait_bounded(&bar[bb], (unsigned)((posted[bb] - 1) & 1), kStageWaitPolls);
+      for (int j = listed < 2 ? 0 : listed - 2; j < listed; ++j)  // (a phase that completed
+        tma::mbar_wait_bounded(&list_bar[j & 1], (unsigned)(j >> 1) & 1u,  // returns at once)
+                               kStageWaitPolls);
+      for (int j = posted < 2 ? 0 : posted - 2; j < posted; ++j)
+        tma::mbar_wait_bounded(&bar[j & 1], (unsigned)(j >> 1) & 1u, kStageWaitPolls);
       return;
     }
   }
@@ -1098,26 +1188,33 @@ template <int D, bool SECOND>
 __device__ __forceinline__ prim<float, D> recon(const workspace &w, const float4 *pk, int c,
                                                 const float *dx, bool swap) {
   float g[4 * layout<D>::GRAD4];
-  if (SECOND) load_grads<D>(w.grads, c, g);
+  if (SECOND) load_grads<D>(w.grads, w.nc, c, g);
   return recon_from<D, SECOND>(load_pack<D>(pk, c), g, dx, swap);
 }
 
 // Area-scaled flux of face f in its own orientation (cells(f)[0] -> [1]),
 // F[k] = RN(flux_k * A_f).  Both cells of a face and the face kernel get the
 // same bits from it.
-template <int D, int KIND, bool SECOND>
+//
+// STREAM: the face's geometry is read once by the launch, so it is marked to
+// leave the caches first, ahead of the packs and gradients (2D face_flux 40.4 ->
+// 38.4 us at 1024^2; where each face is read twice, in flux_update, it costs 15 %,
+// and in 3D 1 %).
+template <int D, int KIND, bool SECOND, bool STREAM = false>
 __device__ __forceinline__ void face_flux_area(const fvh_mesh_view &m, const workspace &w,
                                                const float4 *__restrict__ pk, int f, int swap,
                                                int outflow, float *F) {
-  const int2 cc = reinterpret_cast<const int2 *>(m.face_cells)[f];
+  const int2 *fc = reinterpret_cast<const int2 *>(m.face_cells) + f;
+  const int2 cc = STREAM ? __ldcs(fc) : *fc;
   float n[D], area;
-  face_geo<D>(w, f, n, area);
+  face_geo<D, STREAM>(w, f, n, area);
   float dx0[D], dx1[D];
   if (D == 2) {
-    const float4 t = w.fdx[f];
+    const float4 t = STREAM ? __ldcs(w.fdx + f) : w.fdx[f];
     dx0[0] = t.x; dx0[1] = t.y; dx1[0] = t.z; dx1[1] = t.w;
   } else {
-    const float4 a = w.fdx[2 * (size_t)f], b = w.fdx[2 * (size_t)f + 1];
+    float4 a, b;
+    ldg256(w.fdx + 2 * (size_t)f, a, b);
     dx0[0] = a.x; dx0[1] = a.y; dx0[D - 1] = a.z;
     dx1[0] = b.x; dx1[1] = b.y; dx1[D - 1] = b.z;
   }
@@ -1190,21 +1287,7 @@ __device__ __forceinline__ void cell_update(const fvh_state_view &s, const works
   }
   float pv[4 * L4];  // predictor increments: (d rho, d v.., d e) as (hi, lo) pairs
   if (STAGE == 1) {
-    const float4 *dp = w.delta + (size_t)L4 * c;
-    float4 t[L4];
-    if (L4 == 2) {
-      ldg256(dp, t[0], t[1]);
-    } else {
-#pragma unroll
-      for (int q = 0; q < L4; ++q) t[q] = dp[q];
-    }
-#pragma unroll
-    for (int q = 0; q < L4; ++q) {
-      pv[4 * q] = t[q].x;
-      pv[4 * q + 1] = t[q].y;
-      pv[4 * q + 2] = t[q].z;
-      pv[4 * q + 3] = t[q].w;
-    }
+    load_planes<L4>(w.delta, w.nc, c, pv);
     rho = df_add(rho, {pv[0], pv[1]});
 #pragma unroll
     for (int i = 0; i < D; ++i) v[i] = df_add(v[i], {pv[2 + 2 * i], pv[3 + 2 * i]});
@@ -1212,16 +1295,17 @@ __device__ __forceinline__ void cell_update(const fvh_state_view &s, const works
   }
   const df rho2 = df_add(rho, du[0]);
   const float r = __frcp_rn(rho2.hi);
-  df k0 = {0.f, 0.f}, dv[D];
+  // (sums start from their first term: 0 + x is x for a normalised x)
+  df k0 = df_mul(v[0], v[0]), dv[D];
 #pragma unroll
   for (int i = 0; i < D; ++i) {
-    k0 = df_add(k0, df_mul(v[i], v[i]));
+    if (i > 0) k0 = df_add(k0, df_mul(v[i], v[i]));
     dv[i] = df_div(df_sub(du[1 + i], df_mul(v[i], du[0])), rho2, r);
   }
   df de = df_div(df_sub(du[D + 1], df_mul(df_add(e, df_half(k0)), du[0])), rho2, r);
-  df vdv = {0.f, 0.f}, dv2 = {0.f, 0.f};
+  df vdv = df_mul(v[0], dv[0]), dv2 = df_mul(dv[0], dv[0]);
 #pragma unroll
-  for (int i = 0; i < D; ++i) {
+  for (int i = 1; i < D; ++i) {
     vdv = df_add(vdv, df_mul(v[i], dv[i]));
     dv2 = df_add(dv2, df_mul(dv[i], dv[i]));
   }
@@ -1242,14 +1326,7 @@ __device__ __forceinline__ void cell_update(const fvh_state_view &s, const works
     t[2 * D + 3] = de.lo;
 #pragma unroll
     for (int q = 2 * D + 4; q < 4 * L4; ++q) t[q] = 0.f;
-    float4 *dp = w.delta + (size_t)L4 * c;
-    if (L4 == 2) {
-      stg256(dp, make_float4(t[0], t[1], t[2], t[3]), make_float4(t[4], t[5], t[6], t[7]));
-    } else {
-#pragma unroll
-      for (int q = 0; q < L4; ++q)
-        dp[q] = make_float4(t[4 * q], t[4 * q + 1], t[4 * q + 2], t[4 * q + 3]);
-    }
+    store_planes<L4>(w.delta, w.nc, c, t);
     float vf[D];
 #pragma unroll
     for (int i = 0; i < D; ++i) vf[i] = df_add(v[i], dv[i]).hi;
@@ -1417,16 +1494,12 @@ template <int D, int KIND, bool SECOND, int BS>
 __global__ void __launch_bounds__(BS, 1024 / BS)
 face_flux_kernel(const fvh_mesh_view m, workspace w, const float4 *__restrict__ pk_in, int swap,
                  int outflow, int rev) {
-  constexpr int F4 = layout<D>::FLUX4;
   for (int i = blockIdx.x * BS + threadIdx.x; i < m.num_faces; i += gridDim.x * BS) {
     const int f = rev ? m.num_faces - 1 - i : i;
-    float F[4 * F4];
-    face_flux_area<D, KIND, SECOND>(m, w, pk_in, f, swap, outflow, F);
-#pragma unroll
-    for (int k = D + 2; k < 4 * F4; ++k) F[k] = 0.f;
-#pragma unroll
-    for (int q = 0; q < F4; ++q)
-      w.fflux[(size_t)F4 * f + q] = make_float4(F[4 * q], F[4 * q + 1], F[4 * q + 2], F[4 * q + 3]);
+    float F[D + 2];
+    face_flux_area<D, KIND, SECOND, D == 2>(m, w, pk_in, f, swap, outflow, F);
+    w.fflux[f] = make_float4(F[0], F[1], F[2], F[3]);
+    if (D == 3) w.fflux5[f] = F[D + 1];
   }
 }
 
@@ -1437,7 +1510,6 @@ gather_update_kernel(const fvh_mesh_view m, const fvh_state_view s, workspace w,
                      float4 *__restrict__ pk_out, const problem_map pm,
                      const update_consts uc, int rev, const next_dt nd,
                      const fvh_state_view out, int has_out) {
-  constexpr int F4 = layout<D>::FLUX4;
   stage_dt sdt;
   float dt_inv = 0.f;
   for (int i = blockIdx.x * BS + threadIdx.x; i < m.num_cells; i += gridDim.x * BS) {
@@ -1449,24 +1521,26 @@ gather_update_kernel(const fvh_mesh_view m, const fvh_state_view s, workspace w,
       continue;
     }
     float shi[D + 2], slo[D + 2];
-#pragma unroll
-    for (int k = 0; k < D + 2; ++k) shi[k] = slo[k] = 0.f;
     const int q0 = m.cell_face_offsets[c], nq = m.cell_face_offsets[c + 1] - q0;
-    for (int k = 0; k < nq; ++k) {
+    auto face = [&](int k, bool first) {
       const int sf = m.cell_faces[q0 + k];
       const int f = sf < 0 ? ~sf : sf;
-      float F[4 * F4];
+      const float4 t = w.fflux[f];
+      float F[D + 2] = {t.x, t.y, t.z, t.w};
+      if (D == 3) F[D + 1] = w.fflux5[f];
 #pragma unroll
-      for (int r = 0; r < F4; ++r) {
-        const float4 t = w.fflux[(size_t)F4 * f + r];
-        F[4 * r] = t.x;
-        F[4 * r + 1] = t.y;
-        F[4 * r + 2] = t.z;
-        F[4 * r + 3] = t.w;
+      for (int k = 0; k < D + 2; ++k) {
+        const float x = sf >= 0 ? -F[k] : F[k];
+        if (first) {
+          shi[k] = x;
+          slo[k] = 0.f;
+        } else {
+          two_sum_acc(shi[k], slo[k], x);
+        }
       }
-#pragma unroll
-      for (int k = 0; k < D + 2; ++k) two_sum_acc(shi[k], slo[k], sf >= 0 ? -F[k] : F[k]);
-    }
+    };
+    face(0, true);  // (a cell has faces; its first flux is the sum so far)
+    for (int k = 1; k < nq; ++k) face(k, false);
     float vn[D], an;
     cell_update<D, STAGE>(s, w, pk_out, pm, c, pr, sdt.dts, shi, slo, uc, vn, &an,
                           STAGE == 1 && has_out ? &out : nullptr);
@@ -1569,10 +1643,11 @@ cudaError_t debug_split(const double *x, int64_t n, float *hi, float *lo, float 
 template <int D>
 static size_t bytes_for(int nc, int nf, int nv) {
   using L = layout<D>;
-  return sizeof(float4) * ((size_t)nc * (2 * L::PACK4 + L::GRAD4 + L::CEN4) + (size_t)nv * L::CEN4 +
-                           (size_t)nf * (L::FGEO4 + L::FDX4 + L::FLUX4) + (size_t)nc * L::DEL4) +
+  return sizeof(float4) * ((size_t)nc * (2 * L::PACK4 + L::GRAD4 + L::CEN4 + L::LSQ4) + (size_t)nv * L::CEN4 +
+                           (size_t)nf * (L::FGEO4 + L::FDX4 + 1) + (size_t)nc * L::DEL4) +
          2 * sizeof(float) * (size_t)nc +
-         256 * 18;  // alignment of each carved array + counters
+         (D == 3 ? sizeof(float) * (size_t)nf : 0) +
+         256 * 20;  // alignment of each carved array + counters
 }
 
 template <int D>
@@ -1589,9 +1664,11 @@ static void carve(workspace *w) {
   w->grads = reinterpret_cast<float4 *>(take(sizeof(float4) * (size_t)w->nc * L::GRAD4));
   w->ccen = reinterpret_cast<float4 *>(take(sizeof(float4) * (size_t)w->nc * L::CEN4));
   w->vcoord = reinterpret_cast<float4 *>(take(sizeof(float4) * (size_t)w->nv * L::CEN4));
+  w->lsq = reinterpret_cast<float4 *>(take(sizeof(float4) * (size_t)w->nc * L::LSQ4));
   w->fgeo = reinterpret_cast<float4 *>(take(sizeof(float4) * (size_t)w->nf * L::FGEO4));
   w->fdx = reinterpret_cast<float4 *>(take(sizeof(float4) * (size_t)w->nf * L::FDX4));
-  w->fflux = reinterpret_cast<float4 *>(take(sizeof(float4) * (size_t)w->nf * L::FLUX4));
+  w->fflux = reinterpret_cast<float4 *>(take(sizeof(float4) * (size_t)w->nf));
+  if (D == 3) w->fflux5 = reinterpret_cast<float *>(take(sizeof(float) * (size_t)w->nf));
   w->delta = reinterpret_cast<float4 *>(take(sizeof(float4) * (size_t)w->nc * L::DEL4));
   w->inv_vol32 = reinterpret_cast<float *>(take(sizeof(float) * (size_t)w->nc));
   w->inv_vol_lo = reinterpret_cast<float *>(take(sizeof(float) * (size_t)w->nc));
@@ -1604,6 +1681,7 @@ static cudaError_t setup_d(const fvh_mesh_view &m, workspace *w, cudaStream_t st
   const int t = 256;
   setup_cells<D><<<(m.num_cells + t - 1) / t, t, 0, st>>>(m, *w);
   setup_vertices<D><<<(m.num_vertices + t - 1) / t, t, 0, st>>>(m, *w);
+  if (D == 3) setup_lsq<<<(m.num_cells + t - 1) / t, t, 0, st>>>(m, *w);
   setup_faces<D><<<(m.num_faces + t - 1) / t, t, 0, st>>>(m, *w);
   return cudaGetLastError();
 }
@@ -1710,6 +1788,9 @@ static unsigned spread_bits16(unsigned x) {
   x = (x | (x << 1)) & 0x55555555u;
   return x;
 }
+
+// Shared memory of a block: two stage buffers and two lists.
+static int stage_smem(const stage_tables &t) { return 2 * t.stage_bytes + 32 * t.list_slots; }
 
 static cudaError_t setup_stage_host(workspace *w, const fvh_mesh_view &m) {
   const int nc = m.num_cells;
@@ -1821,29 +1902,31 @@ static cudaError_t setup_stage_host(workspace *w, const fvh_mesh_view &m) {
   if (t.stage_bytes > kStageMaxBytes) return cudaSuccess;
   std::vector<int> cells((size_t)nchunks * kStageCells, -1);
   for (int i = 0; i < nc; ++i) cells[i] = order[i].second;
-  std::vector<int> run_off(nchunks + 1, 0);
-  std::vector<long long> topo_off(nchunks + 1, 0);
-  std::vector<unsigned> chunk_bytes(nchunks, 0);
+  size_t most = 0, units = 0;
+  for (int k = 0; k < nchunks; ++k) most = std::max(most, runs[k].size());
+  t.list_slots = (int)most + 1;
+  std::vector<stage_list> lists((size_t)nchunks * t.list_slots);
   for (int k = 0; k < nchunks; ++k) {
-    run_off[k + 1] = run_off[k] + (int)runs[k].size();
-    topo_off[k + 1] = topo_off[k] + 4 * (long long)topo[k].size();
-    chunk_bytes[k] = 4 * (unsigned)topo[k].size();
-    for (const stage_run &r : runs[k]) chunk_bytes[k] += (unsigned)r.count * (r.kind == 0 ? 48u : 16u);
+    stage_list *l = lists.data() + (size_t)k * t.list_slots;
+    l->head = {(int)runs[k].size(), 4 * (unsigned)topo[k].size(), (unsigned)units,
+               (unsigned)(topo[k].size() / 4)};
+    for (size_t r = 0; r < runs[k].size(); ++r) {
+      l[1 + r].run = runs[k][r];
+      l->head.bytes += (unsigned)runs[k][r].count * (runs[k][r].kind == 0 ? 48u : 16u);
+    }
+    units += topo[k].size() / 4;
   }
-  std::vector<stage_run> all(run_off[nchunks]);
-  std::vector<unsigned> blob(topo_off[nchunks] / 4);
-  for (int k = 0; k < nchunks; ++k) {
-    std::copy(runs[k].begin(), runs[k].end(), all.begin() + run_off[k]);
-    std::copy(topo[k].begin(), topo[k].end(), blob.begin() + topo_off[k] / 4);
-  }
+  if (t.stage_bytes + 16 * t.list_slots > kStageMaxBytes || units > UINT32_MAX) return cudaSuccess;
+  std::vector<unsigned> blob(4 * units);
+  for (int k = 0; k < nchunks; ++k)
+    std::copy(topo[k].begin(), topo[k].end(),
+              blob.begin() + 4 * (size_t)lists[(size_t)k * t.list_slots].head.topo_at);
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-  const size_t b_cells = up(sizeof(int) * cells.size()), b_off = up(sizeof(int) * run_off.size()),
-               b_runs = up(sizeof(stage_run) * all.size()),
-               b_toff = up(sizeof(long long) * topo_off.size()),
-               b_topo = up(sizeof(unsigned) * blob.size()),
-               b_bytes = up(sizeof(unsigned) * chunk_bytes.size());
+  const size_t b_cells = up(sizeof(int) * cells.size()),
+               b_lists = up(sizeof(stage_list) * lists.size()),
+               b_topo = up(sizeof(unsigned) * blob.size());
   char *base = nullptr;
-  e = cudaMalloc(&base, b_cells + b_off + b_runs + b_toff + b_topo + b_bytes);
+  e = cudaMalloc(&base, b_cells + b_lists + b_topo);
   if (e != cudaSuccess) return e;
   w->stage_base = base;
   char *p = base;
@@ -1855,16 +1938,12 @@ static cudaError_t setup_stage_host(workspace *w, const fvh_mesh_view &m) {
   };
   t.nchunks = nchunks;
   t.cells = reinterpret_cast<const int *>(put(cells.data(), sizeof(int) * cells.size(), b_cells));
-  t.run_off = reinterpret_cast<const int *>(put(run_off.data(), sizeof(int) * run_off.size(), b_off));
-  t.runs = reinterpret_cast<const stage_run *>(put(all.data(), sizeof(stage_run) * all.size(), b_runs));
-  t.topo_off = reinterpret_cast<const long long *>(
-      put(topo_off.data(), sizeof(long long) * topo_off.size(), b_toff));
+  t.lists = reinterpret_cast<const stage_list *>(
+      put(lists.data(), sizeof(stage_list) * lists.size(), b_lists));
   t.topo = reinterpret_cast<const unsigned *>(put(blob.data(), sizeof(unsigned) * blob.size(), b_topo));
-  t.bytes = reinterpret_cast<const unsigned *>(
-      put(chunk_bytes.data(), sizeof(unsigned) * chunk_bytes.size(), b_bytes));
   if (e != cudaSuccess) return e;
   // persistent grid: the blocks that fit on the device at once
-  const int smem = 2 * t.stage_bytes;
+  const int smem = stage_smem(t);
   e = cudaFuncSetAttribute(gradients_staged_kernel<true>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e == cudaSuccess)
@@ -1938,7 +2017,7 @@ static void launch_stage_bs(workspace *w, const fvh_mesh_view &m, const fvh_para
   if (SECOND) {
     dir ^= 1;
     if (D == 2 && staged && w->stage.nchunks > 0 && !pm.cell_problem) {
-      const int smem = 2 * w->stage.stage_bytes;
+      const int smem = stage_smem(w->stage);
       if (p.limiter == FVH_LIMITER_NONE)
         gradients_staged_kernel<false><<<w->stage_blocks, kStageCells, smem, st>>>(
             m, *w, pk_in, w->stage, dir, pm.status);

@@ -1942,13 +1942,15 @@ static cudaError_t setup_stage_host(workspace *w, const fvh_mesh_view &m) {
       put(lists.data(), sizeof(stage_list) * lists.size(), b_lists));
   t.topo = reinterpret_cast<const unsigned *>(put(blob.data(), sizeof(unsigned) * blob.size(), b_topo));
   if (e != cudaSuccess) return e;
-  // persistent grid: the blocks that fit on the device at once
-  const int smem = stage_smem(t);
+  // The kernel's limit is the most any mesh may stage, not this mesh's need: it
+  // is one setting for all solvers.
+  const int smem = stage_smem(t), most_smem = 2 * kStageMaxBytes;
   e = cudaFuncSetAttribute(gradients_staged_kernel<true>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, most_smem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(gradients_staged_kernel<false>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, most_smem);
+  // persistent grid: the blocks that fit on the device at once
   int per_sm = 0, dev = 0, sms = 0;
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gradients_staged_kernel<true>,

@@ -140,8 +140,18 @@ __device__ __forceinline__ void stg256(float4 *p, float4 a, float4 b) {
                : "memory");
 }
 
+// one 32-byte load (p 32-byte aligned) of what an earlier kernel of the step
+// wrote; volatile keeps it behind after_previous
+__device__ __forceinline__ void ld256(const float4 *p, float4 &a, float4 &b) {
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z),
+                 "=f"(b.w)
+               : "l"(p));
+}
+
 // one 32-byte load through the read-only path (sm_100+ 256-bit vector load);
-// p must be 32-byte aligned and not written during the kernel
+// p must be 32-byte aligned and written by no kernel of a step: a kernel may be
+// resident before its predecessor has ended (fvh::launch)
 __device__ __forceinline__ void ldg256(const float4 *p, float4 &a, float4 &b) {
   asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
       : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
@@ -152,9 +162,9 @@ __device__ __forceinline__ void ldg256(const float4 *p, float4 &a, float4 &b) {
 //   2D: f4[0] = (d, vx, vy, p)  f4[1] = (e, a, 0, 0)
 //   3D: f4[0] = (d, vx, vy, vz) f4[1] = (p, e, a, 0)
 template <int D>
-__device__ __forceinline__ prim<float, D> load_pack(const float4 *pk, int c) {
+__device__ __forceinline__ prim<float, D> load_pack(const float4 *__restrict__ pk, int c) {
   float4 a, b;
-  ldg256(pk + 2 * (size_t)c, a, b);
+  ld256(pk + 2 * (size_t)c, a, b);
   prim<float, D> w;
   w.d = a.x;
   w.v[0] = a.y;
@@ -187,7 +197,7 @@ template <int N4>
 __device__ __forceinline__ void load_planes(const float4 *base, int n, int c, float *x) {
   float4 t[N4];
 #pragma unroll
-  for (int q = 0; q + 1 < N4; q += 2) ldg256(base + (size_t)q * n + 2 * (size_t)c, t[q], t[q + 1]);
+  for (int q = 0; q + 1 < N4; q += 2) ld256(base + (size_t)q * n + 2 * (size_t)c, t[q], t[q + 1]);
   if (N4 % 2) t[N4 - 1] = base[(size_t)(N4 - 1) * n + c];
 #pragma unroll
   for (int q = 0; q < N4; ++q) {
@@ -951,6 +961,7 @@ __device__ __forceinline__ void cell_gradients_pairs(const workspace &w, int c0,
 template <int D, bool LIMIT, int BS>
 __global__ void __launch_bounds__(BS, (D == 2 ? 1024 : 640) / BS)
 gradients_kernel(const fvh_mesh_view m, workspace w, const float4 *__restrict__ pk, int rev) {
+  after_previous();
   for (int i = blockIdx.x * BS + threadIdx.x; i < m.num_cells; i += gridDim.x * BS) {
     const int c0 = rev ? m.num_cells - 1 - i : i;
     float xh[3], xl[3];
@@ -962,12 +973,12 @@ gradients_kernel(const fvh_mesh_view m, workspace w, const float4 *__restrict__ 
     };
     if (D == 2) {
       float4 a0, b0;
-      ldg256(pk + 2 * (size_t)c0, a0, b0);
+      ld256(pk + 2 * (size_t)c0, a0, b0);
       cell_gradients_pairs<D, LIMIT, 4>(
           w, c0, a0, b0, xh, xl, nn,
           [&](int q, float4 &a, float4 &b, float *yh, float *yl) {
             const int c1 = m.cell_nbrs[q0 + q];
-            ldg256(pk + 2 * (size_t)c1, a, b);
+            ld256(pk + 2 * (size_t)c1, a, b);
             load_cen<D>(w.ccen, c1, yh, yl);
           },
           nr, vtx);
@@ -984,6 +995,7 @@ gradients_kernel(const fvh_mesh_view m, workspace w, const float4 *__restrict__ 
           nr, vtx);
     }
   }
+  let_next_start();
 }
 
 // ---------------------------------------------------------------------------
@@ -1076,6 +1088,9 @@ gradients_staged_kernel(const fvh_mesh_view m, workspace w, const float4 *__rest
   if (mine > 0) {
     fetch_list(chunk_of(0), 0);
     if (mine > 1) fetch_list(chunk_of(1), 1);
+  }
+  after_previous();
+  if (mine > 0) {
     if (tid < 32) {
       landed = __all_sync(0xffffffffu, tma::mbar_wait_bounded(&list_bar[0], 0u, kStageWaitPolls));
       if (landed) post(0);
@@ -1088,6 +1103,7 @@ gradients_staged_kernel(const fvh_mesh_view m, workspace w, const float4 *__rest
     const unsigned phase = (unsigned)(it >> 1) & 1u;
     const int k = chunk_of(it);
     const int c0 = c_ahead;
+    if (it + 1 == mine) let_next_start();
     // buffers b ^ 1 were last read during the previous chunk (lists: at its
     // start), before the barrier that ended it
     if (it + 1 < mine) {
@@ -1160,7 +1176,7 @@ gradients_staged_kernel(const fvh_mesh_view m, workspace w, const float4 *__rest
 // ---------------------------------------------------------------------------
 // reconstruct the state of cell c at offset dx (x_f - x_c) from pack + grads
 template <int D, bool SECOND>
-__device__ __forceinline__ prim<float, D> recon(const workspace &w, const float4 *pk, int c,
+__device__ __forceinline__ prim<float, D> recon(const workspace &w, const float4 *__restrict__ pk, int c,
                                                 const float *dx, bool swap);
 
 // reconstruction of cell values u (pack) with gradients g at offset dx
@@ -1169,15 +1185,16 @@ __device__ __forceinline__ prim<float, D> recon_from(prim<float, D> u, const flo
                                                      const float *dx, bool swap) {
   if (SECOND) {
     // gradient rows: 0 d, 1..D v, D+1 e, D+2 p, D+3 a
-    const int ge = swap ? D + 2 : D + 1;  // row added to the energy slot
-    const int gp = swap ? D + 1 : D + 2;  // row added to the pressure slot
 #pragma unroll
     for (int i = 0; i < D; ++i) {
       u.d += dx[i] * g[0 * D + i];
 #pragma unroll
       for (int d = 0; d < D; ++d) u.v[d] += dx[i] * g[(1 + d) * D + i];
-      u.p += dx[i] * g[gp * D + i];
-      u.e += dx[i] * g[ge * D + i];
+      // (selected by value: an index known only at run time puts the record in
+      // local memory; 3D face_flux 160 -> 127 us at 128^3, flux_update 446 -> 276)
+      const float ge = g[(D + 1) * D + i], gp = g[(D + 2) * D + i];
+      u.p += dx[i] * (swap ? ge : gp);
+      u.e += dx[i] * (swap ? gp : ge);
       u.a += dx[i] * g[(D + 3) * D + i];
     }
   }
@@ -1185,7 +1202,7 @@ __device__ __forceinline__ prim<float, D> recon_from(prim<float, D> u, const flo
 }
 
 template <int D, bool SECOND>
-__device__ __forceinline__ prim<float, D> recon(const workspace &w, const float4 *pk, int c,
+__device__ __forceinline__ prim<float, D> recon(const workspace &w, const float4 *__restrict__ pk, int c,
                                                 const float *dx, bool swap) {
   float g[4 * layout<D>::GRAD4];
   if (SECOND) load_grads<D>(w.grads, w.nc, c, g);
@@ -1456,6 +1473,7 @@ flux_update_kernel(const fvh_mesh_view m, const fvh_state_view s, workspace w,
                    int rev, const next_dt nd, const fvh_state_view out, int has_out) {
   // Reads pk_in (all cells) and the cell's own FP64 state; the predictor writes
   // the cell's increments and pk_out record, the corrector its FP64 state.
+  after_previous();
   stage_dt sdt;
   float dt_inv = 0.f;
   for (int i = blockIdx.x * BS + threadIdx.x; i < m.num_cells; i += gridDim.x * BS) {
@@ -1486,14 +1504,18 @@ flux_update_kernel(const fvh_mesh_view m, const fvh_state_view s, workspace w,
     if (NEXT == 2) dt_inv = smax(cell_cfl<D>(m, w, c, vn, an), dt_inv);
     if (NEXT == 3) problem_cfl(pm, pr, cell_cfl<D>(m, w, c, vn, an));
   }
+  let_next_start();
   if (NEXT == 2) finish_cfl(w, nd, dt_inv);
 }
 
 // Face schedule, part 1: one flux per face into the FP32 face-flux array.
+// 2D: 1280 threads per SM (35.6 us a launch at 1024^2 against 36.9 with 1024), 3D
+// 1024 (128^3 126.5 us, with 1280 132.6, with 768 140.5).
 template <int D, int KIND, bool SECOND, int BS>
-__global__ void __launch_bounds__(BS, 1024 / BS)
+__global__ void __launch_bounds__(BS, (D == 2 ? 1280 : 1024) / BS)
 face_flux_kernel(const fvh_mesh_view m, workspace w, const float4 *__restrict__ pk_in, int swap,
                  int outflow, int rev) {
+  after_previous();
   for (int i = blockIdx.x * BS + threadIdx.x; i < m.num_faces; i += gridDim.x * BS) {
     const int f = rev ? m.num_faces - 1 - i : i;
     float F[D + 2];
@@ -1501,15 +1523,20 @@ face_flux_kernel(const fvh_mesh_view m, workspace w, const float4 *__restrict__ 
     w.fflux[f] = make_float4(F[0], F[1], F[2], F[3]);
     if (D == 3) w.fflux5[f] = F[D + 1];
   }
+  let_next_start();
 }
 
 // Face schedule, part 2: cell-centric gather of the face-flux array + update.
+// Threads per SM it is compiled for: the predictor 1280 (1024^2 with the staged
+// gradients 251.3 us a step against 253.3 with 1024, 3D 128^3 1002 against 1005),
+// the corrector 1024 (896: 270.7).
 template <int D, int BS, int STAGE, int NEXT = 0>
-__global__ void __launch_bounds__(BS, 1024 / BS)
+__global__ void __launch_bounds__(BS, (STAGE == 0 ? 1280 : 1024) / BS)
 gather_update_kernel(const fvh_mesh_view m, const fvh_state_view s, workspace w,
                      float4 *__restrict__ pk_out, const problem_map pm,
                      const update_consts uc, int rev, const next_dt nd,
                      const fvh_state_view out, int has_out) {
+  after_previous();
   stage_dt sdt;
   float dt_inv = 0.f;
   for (int i = blockIdx.x * BS + threadIdx.x; i < m.num_cells; i += gridDim.x * BS) {
@@ -1547,6 +1574,7 @@ gather_update_kernel(const fvh_mesh_view m, const fvh_state_view s, workspace w,
     if (NEXT == 2) dt_inv = smax(cell_cfl<D>(m, w, c, vn, an), dt_inv);
     if (NEXT == 3) problem_cfl(pm, pr, cell_cfl<D>(m, w, c, vn, an));
   }
+  let_next_start();
   if (NEXT == 2) finish_cfl(w, nd, dt_inv);
 }
 
@@ -1560,6 +1588,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS)
 face_colour_kernel(const fvh_mesh_view m, workspace w, const float4 *__restrict__ pk_in,
                    int swap, int outflow, int first, int count) {
   constexpr int NQ = D + 2;
+  after_previous();
   for (int i = blockIdx.x * BS + threadIdx.x; i < count; i += gridDim.x * BS) {
     const int f = w.colour_faces[first + i];
     float F[NQ];
@@ -1590,6 +1619,7 @@ colour_update_kernel(const fvh_mesh_view m, const fvh_state_view s, workspace w,
                      const update_consts uc, int rev, const next_dt nd,
                      const fvh_state_view out, int has_out) {
   constexpr int NQ = D + 2;
+  after_previous();
   stage_dt sdt;
   float dt_inv = 0.f;
   for (int i = blockIdx.x * BS + threadIdx.x; i < m.num_cells; i += gridDim.x * BS) {
@@ -1612,6 +1642,7 @@ colour_update_kernel(const fvh_mesh_view m, const fvh_state_view s, workspace w,
                           STAGE == 1 && has_out ? &out : nullptr);
     if (NEXT == 2) dt_inv = smax(cell_cfl<D>(m, w, c, vn, an), dt_inv);
   }
+  let_next_start();
   if (NEXT == 2) finish_cfl(w, nd, dt_inv);
 }
 
@@ -2006,6 +2037,12 @@ static void launch_stage_bs(workspace *w, const fvh_mesh_view &m, const fvh_para
                             int cpt, int schedule, bool staged, cudaStream_t st,
                             const launch_mark &mark,
                             int &dir, const next_dt *nd) {
+  // each kernel starts as its predecessor ends (us a step: KH 64^2 22.7 -> 21.1,
+  // triangles 203x149 36.4 -> 34.8, 3D 64^3 164 -> 162, 40 problems 227 -> 224;
+  // no change from a million cells on).  Not beside the staged gradients, whose
+  // blocks fill every SM: their successor's blocks then settle unevenly (1024^2
+  // 255 -> 261, with flux_update 258 -> 318).
+  const bool overlap = !staged && !mark.fn;
   const long long per = (long long)BS * cpt;
   const int nb = (int)((m.num_cells + per - 1) / per);
   const float4 *pk_in = stage == 0 ? w->pack : w->pack2;
@@ -2021,15 +2058,15 @@ static void launch_stage_bs(workspace *w, const fvh_mesh_view &m, const fvh_para
     if (D == 2 && staged && w->stage.nchunks > 0 && !pm.cell_problem) {
       const int smem = stage_smem(w->stage);
       if (p.limiter == FVH_LIMITER_NONE)
-        gradients_staged_kernel<false><<<w->stage_blocks, kStageCells, smem, st>>>(
-            m, *w, pk_in, w->stage, dir, pm.status);
+        launch_with(smem, gradients_staged_kernel<false>, w->stage_blocks, kStageCells, st, overlap,
+                    m, *w, pk_in, w->stage, dir, pm.status);
       else
-        gradients_staged_kernel<true><<<w->stage_blocks, kStageCells, smem, st>>>(
-            m, *w, pk_in, w->stage, dir, pm.status);
+        launch_with(smem, gradients_staged_kernel<true>, w->stage_blocks, kStageCells, st, overlap, m,
+                    *w, pk_in, w->stage, dir, pm.status);
     } else if (p.limiter == FVH_LIMITER_NONE) {
-      gradients_kernel<D, false, BS><<<nb, BS, 0, st>>>(m, *w, pk_in, dir);
+      launch(gradients_kernel<D, false, BS>, nb, BS, st, overlap, m, *w, pk_in, dir);
     } else {
-      gradients_kernel<D, true, BS><<<nb, BS, 0, st>>>(m, *w, pk_in, dir);
+      launch(gradients_kernel<D, true, BS>, nb, BS, st, overlap, m, *w, pk_in, dir);
     }
     mark("gradients");
   }
@@ -2045,58 +2082,54 @@ static void launch_stage_bs(workspace *w, const fvh_mesh_view &m, const fvh_para
     for (int col = 0; col < w->ncolours; ++col) {
       const int first = w->colour_off[col], count = w->colour_off[col + 1] - first;
       const int nbc = (int)((count + per - 1) / per);
-      face_colour_kernel<D, KIND, SECOND, BS><<<nbc > 0 ? nbc : 1, BS, 0, st>>>(
-          m, *w, pk_in, p.recon_swap_ep, p.boundary, first, count);
+      launch(face_colour_kernel<D, KIND, SECOND, BS>, nbc > 0 ? nbc : 1, BS, st, overlap, m, *w, pk_in,
+             p.recon_swap_ep, p.boundary, first, count);
       mark("face_colour");
     }
     dir ^= 1;
+    auto go = [&](auto kernel, int blocks, int has_out) {
+      launch(kernel, blocks, BS, st, overlap, m, s, *w, pk_out, pm, k, dir, ndv, ndv.out, has_out);
+    };
     if (stage == 0)
-      colour_update_kernel<D, BS, 0><<<nb, BS, 0, st>>>(m, s, *w, pk_out, pm, k, dir, ndv,
-                                                        ndv.out, 0);
+      go(colour_update_kernel<D, BS, 0>, nb, 0);
     else if (next)
-      colour_update_kernel<D, BS, 1, 2><<<nb_next, BS, 0, st>>>(m, s, *w, pk_out, pm, k, dir,
-                                                                 ndv, ndv.out, ndv.has_out);
+      go(colour_update_kernel<D, BS, 1, 2>, nb_next, ndv.has_out);
     else
-      colour_update_kernel<D, BS, 1><<<nb, BS, 0, st>>>(m, s, *w, pk_out, pm, k, dir, ndv,
-                                                        ndv.out, ndv.has_out);
+      go(colour_update_kernel<D, BS, 1>, nb, ndv.has_out);
     mark("colour_update");
   } else if (schedule == 1) {
     const int nbf = (int)((m.num_faces + per - 1) / per);
     dir ^= 1;
-    face_flux_kernel<D, KIND, SECOND, BS><<<nbf, BS, 0, st>>>(m, *w, pk_in, p.recon_swap_ep,
-                                                               p.boundary, dir);
+    launch(face_flux_kernel<D, KIND, SECOND, BS>, nbf, BS, st, overlap, m, *w, pk_in,
+           p.recon_swap_ep, p.boundary, dir);
     mark("face_flux");
     dir ^= 1;
+    auto go = [&](auto kernel, int blocks, int has_out) {
+      launch(kernel, blocks, BS, st, overlap, m, s, *w, pk_out, pm, k, dir, ndv, ndv.out, has_out);
+    };
     if (stage == 0)
-      gather_update_kernel<D, BS, 0><<<nb, BS, 0, st>>>(m, s, *w, pk_out, pm, k, dir, ndv,
-                                                        ndv.out, 0);
+      go(gather_update_kernel<D, BS, 0>, nb, 0);
     else if (next && ndv.batch)
-      gather_update_kernel<D, BS, 1, 3><<<nb, BS, 0, st>>>(m, s, *w, pk_out, pm, k, dir, ndv,
-                                                           ndv.out, ndv.has_out);
+      go(gather_update_kernel<D, BS, 1, 3>, nb, ndv.has_out);
     else if (next)
-      gather_update_kernel<D, BS, 1, 2><<<nb_next, BS, 0, st>>>(m, s, *w, pk_out, pm, k, dir,
-                                                                 ndv, ndv.out, ndv.has_out);
+      go(gather_update_kernel<D, BS, 1, 2>, nb_next, ndv.has_out);
     else
-      gather_update_kernel<D, BS, 1><<<nb, BS, 0, st>>>(m, s, *w, pk_out, pm, k, dir, ndv,
-                                                        ndv.out, ndv.has_out);
+      go(gather_update_kernel<D, BS, 1>, nb, ndv.has_out);
     mark("gather_update");
   } else {
     dir ^= 1;
+    auto go = [&](auto kernel, int blocks, int has_out) {
+      launch(kernel, blocks, BS, st, overlap, m, s, *w, pk_in, pk_out, pm, k, p.recon_swap_ep,
+             p.boundary, dir, ndv, ndv.out, has_out);
+    };
     if (stage == 0)
-      flux_update_kernel<D, KIND, SECOND, BS, 0><<<nb, BS, 0, st>>>(
-          m, s, *w, pk_in, pk_out, pm, k, p.recon_swap_ep, p.boundary, dir, ndv, ndv.out, 0);
+      go(flux_update_kernel<D, KIND, SECOND, BS, 0>, nb, 0);
     else if (next && ndv.batch)
-      flux_update_kernel<D, KIND, SECOND, BS, 1, 3><<<nb, BS, 0, st>>>(
-          m, s, *w, pk_in, pk_out, pm, k, p.recon_swap_ep, p.boundary, dir, ndv, ndv.out,
-          ndv.has_out);
+      go(flux_update_kernel<D, KIND, SECOND, BS, 1, 3>, nb, ndv.has_out);
     else if (next)
-      flux_update_kernel<D, KIND, SECOND, BS, 1, 2><<<nb_next, BS, 0, st>>>(
-          m, s, *w, pk_in, pk_out, pm, k, p.recon_swap_ep, p.boundary, dir, ndv, ndv.out,
-          ndv.has_out);
+      go(flux_update_kernel<D, KIND, SECOND, BS, 1, 2>, nb_next, ndv.has_out);
     else
-      flux_update_kernel<D, KIND, SECOND, BS, 1><<<nb, BS, 0, st>>>(
-          m, s, *w, pk_in, pk_out, pm, k, p.recon_swap_ep, p.boundary, dir, ndv, ndv.out,
-          ndv.has_out);
+      go(flux_update_kernel<D, KIND, SECOND, BS, 1>, nb, ndv.has_out);
     mark("flux_update");
   }
 }

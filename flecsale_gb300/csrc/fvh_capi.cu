@@ -233,8 +233,6 @@ fvh_status fvh_solver_create(const fvh_mesh_view *mesh, const fvh_params *params
     cudaError_t e = cudaSuccess;
     if (params->precision == FVH_PRECISION_FP64) {
       e = cudaMalloc(&s->work, sizeof(double) * (ng * nc + (size_t)(D + 2) * nf));
-      // zero gradients, which a first-order solver keeps
-      if (e == cudaSuccess) e = cudaMemset(s->work, 0, sizeof(double) * ng * nc);
       if (e == cudaSuccess) {
         double *b = s->work;
         for (int i = 0; i < D; ++i, b += nc) s->grads.density[i] = b;
@@ -308,6 +306,12 @@ static fvh_status solver_step_enqueue(fvh_solver *s, const fvh_state_view *state
   const bool overlap = m.num_cells <= kOverlapCells && !mark.fn;
   fvh_status r = FVH_OK;
   if (f.pack_first) {
+    // first order: zero gradients for all steps up to the caller's next call
+    if (p.order == 1) {
+      const size_t ng = (size_t)(m.dim + 4) * m.dim;
+      r = from_cuda(cudaMemsetAsync(s->work, 0, sizeof(double) * ng * m.num_cells, st));
+      if (r != FVH_OK) return r;
+    }
     r = from_cuda(m.dim == 2 ? fvh::plain::launch_dt<2>(m, *state, p, t, dt, partial, nb, s->status,
                                                         st, s->tab.slot_dx, f.src, nd.maximum)
                              : fvh::plain::launch_dt<3>(m, *state, p, t, dt, partial, nb, s->status,
@@ -317,7 +321,7 @@ static fvh_status solver_step_enqueue(fvh_solver *s, const fvh_state_view *state
   for (int stage = 0; stage < 2 && r == FVH_OK; ++stage) {
     // a step that follows another of its run forms dt in its first kernel
     const fvh::plain::next_dt &first = stage == 0 && !f.pack_first ? nd : none;
-    if (p.order != 1) {  // (first order: the gradients stay zero as created)
+    if (p.order != 1) {
       r = from_cuda(m.dim == 2 ? fvh::plain::launch_gradients<2>(m, *state, s->grads, p, st,
                                                                  s->tab, first, overlap)
                                : fvh::plain::launch_gradients<3>(m, *state, s->grads, p, st,

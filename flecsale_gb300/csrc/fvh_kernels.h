@@ -27,8 +27,10 @@ __host__ __device__ inline unsigned long long status_key(long long cell, int cod
 // Before `after_previous` it reads only what no kernel of a step writes (the
 // mesh, the tables); after it, everything the predecessors wrote is visible.
 // Every kernel of a step that may have such a successor calls it, so that a
-// kernel's end implies the end of all before it; `let_next_start` at a kernel's
-// start is what allows the overlap.  Launched without it both do nothing.
+// kernel's end implies the end of all before it.  `let_next_start` comes late in a
+// kernel, when its blocks are about to leave: at its start the successor's blocks
+// take places between its own and land unevenly (64^2 FP64, 10 steps: 536 -> 609
+// us, 144^2 834 -> 1,239).  Launched without overlap both do nothing.
 __device__ __forceinline__ void let_next_start() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

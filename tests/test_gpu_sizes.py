@@ -1,6 +1,8 @@
 """FP64 runs on both sides of every size at which the kernels change form (few
 cells or faces, one variable or two per thread), against the oracle bit for bit:
 a run of three steps carries dt from each corrector to the next step."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -50,3 +52,32 @@ def test_run_bitwise(cuda, oracle_lib, dim, n, order):
     again = dstate.download(stream)
     stream.synchronize()
     assert np.array_equal(again, state)
+
+
+@pytest.mark.parametrize("steps", [1, 10])
+def test_first_order_ignores_what_its_gradients_hold(cuda, oracle_lib, steps):
+    """A first-order solver's gradients are zero in every run and step, also after
+    the caller has filled them through the solver's own view."""
+    mesh = H.HostMesh.box(2, (24, 17), [0, 0], [1, 1], 0.15, 5)
+    p = H.make_params(2, flux="hlle", order=1, cfl=0.3, final_time=1e9)
+    second = H.make_params(2, flux="hlle", order=2, cfl=0.3, final_time=1e9)
+    x = mesh.arrays()["cell_centroid"]
+    state = H.state_from_dvp(2, 1 + (x[0] < 0.5), 0.1 * x, 1 + (x[0] < 0.5))
+    one = state.copy()
+    U.oracle_run(oracle_lib, mesh, state, p, 2 * steps)
+    dmesh, dstate = H.DeviceMesh(mesh), H.DeviceState(2, mesh.num_cells)
+    solver = H.Solver(dmesh, p)
+    stream = cuda.cuda.Stream()
+    dstate.upload(one, stream)
+    solver.reset(0.0, stream)
+    for _ in range(2):
+        H.check(H.lib().fvh_evaluate_gradients(C.byref(dmesh.view), C.byref(dstate.view),
+                                               C.byref(solver.gradients), C.byref(second),
+                                               C.c_void_p(stream.cuda_stream)))
+        if steps == 1:
+            solver.step(dstate, stream)
+        else:
+            solver.run(dstate, steps, stream=stream)
+    out = dstate.download(stream)
+    stream.synchronize()
+    assert np.array_equal(out, state)

@@ -65,6 +65,14 @@ struct fvh_solver {
 // (930 -> 880 us and 2.67 -> 2.51 ms; 64^2 10 steps 541 -> 511 us; no change at
 // 112^2).  On large meshes a launch is lost in its kernel.
 constexpr int kManySteps = 4, kManyStepsCells = 262144, kOverlapCells = 10000;
+// Capturing costs 25 us for a step and 80 us for a run.  The first call on a state
+// launches its kernels one by one while that is cheaper: overlapped launches follow one
+// another about as fast as in a graph (us on new states, one by one and captured:
+// mixed 32x32 a step 36 and 60, 8 steps 182 and 260, 20 steps 421 and 497, 64 steps
+// 1,295 and 1,357; FP64 32x32 64 steps 2,590 and 2,678), the others some 10 us a step
+// slower (FP64 200x200 8 steps 976 and 955, 20 steps 2,415 and 2,231).  A second call
+// on the same state captures (mixed 32x32 then 32 us a step).
+constexpr int64_t kCaptureSteps = 128, kCaptureStepsApart = 8;
 
 static void drop_graphs(fvh_solver *s) {
   for (auto &g : s->graph)
@@ -603,18 +611,32 @@ fvh_status fvh_solver_profile(fvh_solver *s, const fvh_state_view *state, int32_
   });
 }
 
+// Whether the graphs are those of this state (a state's pointers are in them);
+// if not, they become its.
+static bool same_state(fvh_solver *s, const fvh_state_view *state) {
+  if (std::memcmp(&s->graph_state, state, sizeof(*state)) == 0) return true;
+  drop_graphs(s);
+  s->graph_state = *state;
+  return false;
+}
+
+// (nothing is built in a stream under capture)
+static bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (st == nullptr) return false;
+  return cudaStreamIsCapturing(st, &c) != cudaSuccess || c != cudaStreamCaptureStatusNone;
+}
+
 // One step is a fixed sequence of launches; each variant is captured once per
 // state into a CUDA graph and replayed in the caller's stream (the legacy
 // default stream too: the capture runs in a stream of the solver's own).  `steps`
 // > 1: that many inner steps of a run in one graph.
 static fvh_status solver_graph(fvh_solver *s, const fvh_state_view *state, cudaStream_t st,
                                fvh::mixed::step_flags f, int steps) {
-  if (std::memcmp(&s->graph_state, state, sizeof(*state)) != 0) {
-    drop_graphs(s);
-    s->graph_state = *state;
-  }
+  same_state(s, state);
   cudaGraphExec_t &ge = s->graph[steps > 1 ? 4 : (f.pack_first ? 2 : 0) + (f.write_next ? 1 : 0)];
   if (!ge) {
+    if (capturing(st)) return FVH_ERR_CUDA;
     cudaError_t e = cudaSuccess;
     if (!s->capture_stream)
       e = cudaStreamCreateWithFlags(&s->capture_stream, cudaStreamNonBlocking);
@@ -648,7 +670,9 @@ static fvh_status solver_step_flags(fvh_solver *s, const fvh_state_view *state, 
 
 fvh_status fvh_solver_step(fvh_solver *s, const fvh_state_view *state, fvh_stream_t stream) {
   if (!s || !state_ok(state, s->mesh.dim)) return FVH_ERR_INVALID_ARGUMENT;
-  return solver_step_flags(s, state, cs(stream), fvh::mixed::step_flags());
+  cudaStream_t st = cs(stream);
+  if (!same_state(s, state) && !capturing(st)) return solver_step_enqueue(s, state, st);
+  return solver_step_flags(s, state, st, fvh::mixed::step_flags());
 }
 
 fvh_status fvh_solver_check(fvh_solver *s, fvh_stream_t stream, double *soln_time,
@@ -688,6 +712,9 @@ fvh_status fvh_solver_run(fvh_solver *s, const fvh_state_view *state, int64_t ns
   fvh_status r = FVH_OK;
   const double tf = s->params.final_time;
   const double t_stop = tf - 1e-12 * std::fabs(tf);
+  const bool apart = s->params.precision == FVH_PRECISION_FP64 && s->mesh.num_cells > kOverlapCells;
+  const bool graphs = same_state(s, state) || capturing(cs(stream)) ||
+                      nsteps >= (apart ? kCaptureStepsApart : kCaptureSteps);
   while (n < nsteps) {
     if (stop_at_final_time) {
       double t = 0;
@@ -698,10 +725,12 @@ fvh_status fvh_solver_run(fvh_solver *s, const fvh_state_view *state, int64_t ns
                               ? (nsteps - n < check_every ? nsteps - n : check_every)
                               : nsteps - n;
     for (int64_t k = 0; k < chunk && r == FVH_OK;) {
-      const bool many = s->mesh.num_cells <= kManyStepsCells && chunk >= 2 * kManySteps && k > 0 &&
-                        k + kManySteps < chunk;
+      const bool many = graphs && s->mesh.num_cells <= kManyStepsCells &&
+                        chunk >= 2 * kManySteps && k > 0 && k + kManySteps < chunk;
       const int steps = many ? kManySteps : 1;
-      r = solver_graph(s, state, cs(stream), chunk_flags(k, chunk), steps);
+      r = graphs
+              ? solver_graph(s, state, cs(stream), chunk_flags(k, chunk), steps)
+              : solver_step_enqueue(s, state, cs(stream), {}, chunk_flags(k, chunk));
       k += steps;
       if (r == FVH_OK) n += steps;
     }

@@ -81,3 +81,30 @@ def test_first_order_ignores_what_its_gradients_hold(cuda, oracle_lib, steps):
     out = dstate.download(stream)
     stream.synchronize()
     assert np.array_equal(out, state)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("legacy", [False, True])
+def test_graphed_and_plain_launches_agree(cuda, precision, legacy):
+    """Runs on two states in turn (launched as they are, or captured, by the number
+    of steps) and twice on one (captured) give the bits of single steps."""
+    mesh = H.HostMesh.box(2, (24, 17), [0, 0], [1, 1], 0.15, 5)
+    p = H.make_params(2, flux="hllc", cfl=0.3, final_time=1e9, precision=precision)
+    x = mesh.arrays()["cell_centroid"]
+    one = H.state_from_dvp(2, 1 + (x[0] < 0.5), 0.1 * x, 1 + (x[0] < 0.5))
+    dmesh = H.DeviceMesh(mesh)
+    solver = H.Solver(dmesh, p)
+    stream = None if legacy else cuda.cuda.Stream()
+    want = {}
+    states = [H.DeviceState(2, mesh.num_cells) for _ in range(2)]
+    for n in (1, 9, 127, 128):
+        states[0].upload(one, stream)
+        solver.reset(0.0, stream)
+        for _ in range(n):
+            solver.step(states[0], stream)
+        want[n] = states[0].download(stream)
+        for s in (1, 1, 0, 1):
+            states[s].upload(one, stream)
+            solver.reset(0.0, stream)
+            assert solver.run(states[s], n, stream=stream) == n
+            assert np.array_equal(states[s].download(stream), want[n]), (n, s)

@@ -32,12 +32,18 @@
 //
 // Code size: the integer forms inline to tens of instructions per product, so
 // a fully unrolled kernel outgrows the SM's instruction cache and its warps
-// stall on instruction fetch.  The kernels keep their neighbour and vertex
-// loops rolled, evaluate each physical flux once per side (selecting the
-// state instead of branching into copies), and take products, quotients and
-// the FP64 redo of a rare unit in out-of-line calls (2.27 -> 1.77 ms per 2D
-// step on the 1024^2 workload; the pipe balance and the variable groups of
-// the gradients below took it on to 1.49 ms).
+// stall on instruction fetch.  The kernels for many cells keep their neighbour
+// and vertex loops rolled, evaluate each physical flux once per side (selecting
+// the state instead of branching into copies), and take the fluxes' products, the
+// quotients and the FP64 redo of a rare unit in out-of-line calls.  Inlined and
+// unrolled the 1024^2 step took 2.27 ms, so arranged 1.77, with the work below
+// 1.19.
+//
+// What bounds them: with many cells the FP64 pipe, 85-90 % busy in the gradients
+// (their sums; most products and all comparisons are on the integer pipes, which
+// are as full in the fluxes and the update); with few cells the chain of loads and
+// operations of one thread, so those kernels (gradients_few_kernel and the others
+// named so) spread a cell's variables over threads and use the FP64 instructions.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -147,12 +153,11 @@ struct arith_hw {
 
 // Products of a part of a unit's work on the FP64 pipe (the same correctly
 // rounded bits), the rest of the arithmetic as the unit's policy does it: a
-// kernel whose integer pipe is the busier one moves some products back.  In
-// the fluxes kernel (ALU 79 %, FP64 54 % with every product on the integer
-// pipe) the physical flux of one side and the area scaling take the FP64
-// pipe: 2D step 1.573 -> 1.521 ms (with the reconstruction of the right side
-// as well: 1.572, the FP64 pipe then the busier one).  In dt the dot
-// products (1.573 -> 1.568).
+// kernel whose integer pipe is the busier one moves some products back: in the
+// fluxes one side's physical flux and the area scaling, in dt the dot products.
+// Four steps at 1024^2 (HLLC) and two at 80^3 (Rusanov) take 4.739 and 4.033 ms so;
+// with the area scaling on the integer pipe 4.718 and 4.047, the physical flux
+// there 4.723 and 4.050, the normal velocities on the FP64 pipe 4.833 and 4.067.
 template <class A>
 struct fp64_products {
   A &ar;

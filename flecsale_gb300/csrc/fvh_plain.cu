@@ -1209,7 +1209,14 @@ template <int D, bool PRE>
 constexpr int grad_min_blocks() { return PRE ? (D == 2 ? 10 : 8) : (D == 2 ? 7 : 6); }
 template <int D>
 constexpr int update_min_blocks() { return D == 2 ? 10 : 1; }
-// Variables of a cell per thread (blockIdx.y: which).  In pairs the offsets
+// Variables of a cell per thread.  The blocks of a cell's groups of variables
+// follow one another, so the offsets and lists they share come from memory once
+// (1024^2: 255 -> 249 us, with waves 344 -> 338; 32^3 one variable a thread 94 -> 92;
+// a whole sweep over the cells per group moved 732 MB instead of 458 at 1024^2).
+// Sharing by spans of 32 to 1,520 blocks: 249 to 251 and 96 to 100.  Pairs in 3D
+// sweep all cells for one pair and then the next, where the values of 26 neighbours
+// count for more than the offsets (80^3, 2 steps 4.03 ms, side by side 4.07).
+// In pairs the offsets
 // x_nbr - x_c are read and taken apart once for both; one by one gives twice the
 // threads, which wins until the chip is full: 10 steps at 360^2 2.58 ms against
 // 2.68 in pairs, at 512^2 4.71 and 4.71, at 1024^2 (4 steps) 4.97 and 4.74; in
@@ -1218,6 +1225,7 @@ constexpr int update_min_blocks() { return D == 2 ? 10 : 1; }
 // 4.51.  Without tables a thread takes all of them, as it builds the
 // least-squares matrix itself.
 constexpr int kSingleCells2D = 262144, kSingleCells3D = 92160;
+constexpr bool groups_side_by_side(int dim, int group) { return dim == 2 || group == 1; }
 
 template <int D, bool LIMIT, bool PRE, int G>
 __global__ void __launch_bounds__(kCellThreads, grad_min_blocks<D, PRE>())
@@ -1226,12 +1234,13 @@ gradients_kernel(const __grid_constant__ fvh_mesh_view m, const __grid_constant_
                  const __grid_constant__ next_dt nd) {
   after_previous();
   finish_dt(nd);
-  const int c0 = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int NV = D + 4, R = NV % G, NG = PRE ? (NV + G - 1) / G : 1;
+  constexpr bool NEXT_TO = groups_side_by_side(D, G);
+  const int c0 = (NEXT_TO ? blockIdx.x / NG : blockIdx.x) * blockDim.x + threadIdx.x;
   if (c0 >= m.num_cells) return;
-  constexpr int NV = D + 4, R = NV % G;
   double r[lsq_width<D>::value];
   arith_opt ar;
-  int k0 = PRE ? blockIdx.y * G : 0;
+  int k0 = (NEXT_TO ? blockIdx.x % NG : blockIdx.y) * G;
   if (!PRE) lsq_matrix<D>(ar, m, c0, r);
 #pragma unroll 1
   for (; k0 + G <= NV; k0 += PRE ? NV + 1 : G)
@@ -1655,15 +1664,17 @@ cudaError_t launch_gradients(const fvh_mesh_view &m, const fvh_state_view &s,
       lim ? go(gradients_few_kernel<D, true, false>) : go(gradients_few_kernel<D, false, false>);
     return cudaGetLastError();
   }
-  auto go = [&](auto kernel, int groups) {
-    const dim3 grid(blocks_of(m.num_cells, kCellThreads), groups);
+  auto go = [&](auto kernel, int groups, int group_size = 2) {
+    const unsigned nb = blocks_of(m.num_cells, kCellThreads);
+    const dim3 grid = groups_side_by_side(D, group_size) ? dim3(nb * groups) : dim3(nb, groups);
     launch(kernel, grid, kCellThreads, st, overlap, m, s, g, t, nd);
   };
   const int pairs = blocks_of(D + 4, 2);
   if (!pre)
     lim ? go(gradients_kernel<D, true, false, 2>, 1) : go(gradients_kernel<D, false, false, 2>, 1);
   else if (m.num_cells <= (D == 2 ? kSingleCells2D : kSingleCells3D))
-    lim ? go(gradients_kernel<D, true, true, 1>, D + 4) : go(gradients_kernel<D, false, true, 1>, D + 4);
+    lim ? go(gradients_kernel<D, true, true, 1>, D + 4, 1)
+        : go(gradients_kernel<D, false, true, 1>, D + 4, 1);
   else
     lim ? go(gradients_kernel<D, true, true, 2>, pairs) : go(gradients_kernel<D, false, true, 2>, pairs);
   return cudaGetLastError();

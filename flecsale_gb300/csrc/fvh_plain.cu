@@ -39,11 +39,11 @@
 // unrolled the 1024^2 step took 2.27 ms, so arranged 1.77, with the work below
 // 1.19.
 //
-// What bounds them: with many cells the FP64 pipe, 85-90 % busy in the gradients
-// (their sums; most products and all comparisons are on the integer pipes, which
-// are as full in the fluxes and the update); with few cells the chain of loads and
-// operations of one thread, so those kernels (gradients_few_kernel and the others
-// named so) spread a cell's variables over threads and use the FP64 instructions.
+// What bounds them: with many cells the FP64 and the integer pipes, loaded alike
+// (1024^2: FP64 66-79 % busy, ALU 59-64 %; the gradients 85-90 % on a flow with waves
+// everywhere); with few cells the chain of loads and operations of one thread, so
+// those kernels (gradients_few_kernel and the others named so) spread a cell's
+// variables over threads and use the FP64 instructions.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -1212,7 +1212,7 @@ constexpr int update_min_blocks() { return D == 2 ? 10 : 1; }
 // Variables of a cell per thread.  The blocks of a cell's groups of variables
 // follow one another, so the offsets and lists they share come from memory once
 // (1024^2: 255 -> 249 us, with waves 344 -> 338; 32^3 one variable a thread 94 -> 92;
-// a whole sweep over the cells per group moved 732 MB instead of 458 at 1024^2).
+// a whole sweep over the cells per group moved 732 MB instead of 391 at 1024^2).
 // Sharing by spans of 32 to 1,520 blocks: 249 to 251 and 96 to 100.  Pairs in 3D
 // sweep all cells for one pair and then the next, where the values of 26 neighbours
 // count for more than the offsets (80^3, 2 steps 4.03 ms, side by side 4.07).

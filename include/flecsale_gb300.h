@@ -286,7 +286,7 @@ fvh_device_status *fvh_solver_status(fvh_solver *s);
 const fvh_gradient_view *fvh_solver_gradients(fvh_solver *s);
 const fvh_flux_view *fvh_solver_fluxes(fvh_solver *s);
 
-/* Kernel launches one fvh_solver_step makes (the CUDA graph's node count). */
+/* Kernel launches one fvh_solver_step makes (kernel nodes of its CUDA graph). */
 int32_t fvh_solver_launches_per_step(const fvh_solver *s);
 
 /* Launch shape of the mixed form's cell kernels: block 128 or 256, cells per

@@ -46,7 +46,7 @@ struct fvh_solver {
   fvh::plain::tables tab;          // views into `tables`
   double *scalars = nullptr;       // [0] soln time, [1] dt, [2..] dt partials
   fvh_device_status *status = nullptr;
-  unsigned long long *dt_maximum = nullptr;  // FP64 form: plain::next_dt::maximum
+  unsigned long long *dt_maximum = nullptr;  // FP64 form: plain::next_dt::maximum, then ::done
   double *host_scalars = nullptr;  // pinned: soln time
   fvh_device_status *host_status = nullptr;
   fvh::mixed::workspace *mixed = nullptr;
@@ -274,10 +274,10 @@ fvh_status fvh_solver_create(const fvh_mesh_view *mesh, const fvh_params *params
     }
     if (e == cudaSuccess)
       e = cudaMalloc(&s->scalars, sizeof(double) * 2 + fvh_time_step_workspace_bytes(mesh->num_cells));
-    // the status word and the FP64 form's carried CFL maximum
-    if (e == cudaSuccess) e = cudaMalloc(&s->status, sizeof(fvh_device_status) + 8);
+    // the status word and the FP64 form's carried CFL maximum with its counter
+    if (e == cudaSuccess) e = cudaMalloc(&s->status, sizeof(fvh_device_status) + 16);
     if (e == cudaSuccess) s->dt_maximum = s->status + 1;
-    if (e == cudaSuccess) e = cudaMemset(s->dt_maximum, 0, 8);
+    if (e == cudaSuccess) e = cudaMemset(s->dt_maximum, 0, 16);
     if (e == cudaSuccess) e = cudaMallocHost(&s->host_scalars, sizeof(double) * 2);
     if (e == cudaSuccess) e = cudaMallocHost(&s->host_status, sizeof(fvh_device_status));
     if (e == cudaSuccess) e = cudaMemset(s->scalars, 0, sizeof(double) * 2);
@@ -310,6 +310,10 @@ static fvh_status solver_step_enqueue(fvh_solver *s, const fvh_state_view *state
   nd.soln_time = t;
   nd.dt = dt;
   nd.status = s->status;
+  nd.partial = partial;
+  nd.nblocks = nb;
+  nd.slot_dx = s->tab.slot_dx;
+  nd.done = reinterpret_cast<unsigned *>(s->dt_maximum + 1);
   const fvh::plain::next_dt none;
   const bool overlap = m.num_cells <= kOverlapCells && !mark.fn;
   fvh_status r = FVH_OK;
@@ -689,6 +693,8 @@ fvh_status fvh_solver_check(fvh_solver *s, fvh_stream_t stream, double *soln_tim
   int64_t cell;
   fvh_status_decode(*s->host_status, &code, &cell);
   if (bad_cell) *bad_cell = cell;
+  // a time that is no number comes of a dt that was none
+  if (code == FVH_OK && std::isnan(s->host_scalars[0])) return FVH_ERR_INFINITE_DT;
   return (fvh_status)code;
 }
 

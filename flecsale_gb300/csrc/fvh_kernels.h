@@ -59,26 +59,27 @@ inline cudaError_t launch(void (*kernel)(P...), dim3 grid, int threads, cudaStre
   return launch_with(0, kernel, grid, threads, st, overlap, args...);
 }
 
-// Block-wide maximum with the reference's std::max semantics; all threads of
-// the block must call it; the result is valid in thread 0.
-__device__ inline double block_max(double v) {
-  __shared__ double warp_max[32];
+// Warp-wide maximum with the reference's std::max semantics; all lanes must
+// call it; the result is valid in lane 0.
+__device__ __forceinline__ double warp_max(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const double w = __shfl_xor_sync(0xffffffffu, v, o);
     v = (v < w) ? w : v;
   }
+  return v;
+}
+// Block-wide maximum likewise; all threads of the block must call it; the
+// result is valid in thread 0.
+__device__ inline double block_max(double v) {
+  __shared__ double warps[32];
+  v = warp_max(v);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) warp_max[warp] = v;
+  if (lane == 0) warps[warp] = v;
   __syncthreads();
   if (warp == 0) {
     const int nw = (blockDim.x + 31) >> 5;
-    v = lane < nw ? warp_max[lane] : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double w = __shfl_xor_sync(0xffffffffu, v, o);
-      v = (v < w) ? w : v;
-    }
+    v = warp_max(lane < nw ? warps[lane] : 0.0);
   }
   return v;
 }
@@ -106,13 +107,20 @@ cudaError_t build_tables(const fvh_mesh_view &m, double *base, int64_t nnz_cf,
 // dt carried from one step of a run to the next: the last update of a step
 // takes the CFL maximum of the new state into *maximum (as the bits of a
 // positive double, cleared when dt is formed), and the first kernel of the next
-// step forms dt from it.  With maximum null neither happens.
+// step forms dt from it.  With maximum null neither happens.  A cell without a
+// number makes *maximum a NaN, and the first fluxes kernel then takes dt from the
+// state as launch_dt does (partial, nblocks: its workspace; slot_dx:
+// tables::slot_dx; done: a counter at zero).
 struct next_dt {
   unsigned long long *maximum = nullptr;
   double cfl = 0, final_time = 0;
   const double *soln_time = nullptr;
   double *dt = nullptr;
   fvh_device_status *status = nullptr;
+  double *partial = nullptr;
+  int nblocks = 0;
+  const double *slot_dx = nullptr;
+  unsigned *done = nullptr;
 };
 
 // overlap (here and below): the kernel may start before its predecessor in the

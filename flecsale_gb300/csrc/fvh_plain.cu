@@ -491,15 +491,89 @@ dt_final_kernel(const double *partial, int nblocks, fvh_params p, const double *
 
 // Inside a run the last update of a step also takes the CFL maximum of the new
 // state (next_dt::maximum, the order of positive doubles is that of their
-// bits), and the first kernel of the following step, which does not read dt,
-// turns it into dt and clears it.
+// bits, and a NaN ranks above them all), and the first kernel of the following
+// step, which does not read dt, turns it into dt and clears it.
+constexpr unsigned long long kInfinity = 0x7ff0000000000000ull;
+__device__ __forceinline__ unsigned block_index() { return blockIdx.y * gridDim.x + blockIdx.x; }
 __device__ __forceinline__ void finish_dt(const next_dt &nd) {
-  if (!nd.maximum || blockIdx.x != 0 || blockIdx.y != 0 || threadIdx.x != 0) return;
-  const double dt_inv = __longlong_as_double((long long)*nd.maximum);
+  if (!nd.maximum || block_index() != 0 || threadIdx.x != 0) return;
+  const unsigned long long max_bits = *nd.maximum;
+  if (max_bits > kInfinity) return;  // (left to redo_dt)
   *nd.maximum = 0ull;
-  write_dt(dt_inv, nd.cfl, nd.final_time, nd.soln_time, nd.dt, nd.status);
+  write_dt(__longlong_as_double((long long)max_bits), nd.cfl, nd.final_time, nd.soln_time, nd.dt,
+           nd.status);
+}
+// Whether it was a NaN, asked in the fluxes kernels by their first nd.nblocks
+// blocks: all of these find the NaN, or a number or the zero it is cleared to.
+__device__ __forceinline__ bool carried_nan(const next_dt &nd) {
+  return nd.maximum && block_index() < (unsigned)nd.nblocks &&
+         *(const volatile unsigned long long *)nd.maximum > kInfinity;
+}
+
+// The maximum of dt_partial_kernel's or dt_final_kernel's block of kDtThreads
+// threads, of which this block, of any whole number of warps, takes one warp
+// after another: value(i) is what its thread i holds.  Valid in thread 0.
+template <class V>
+__device__ __forceinline__ double dt_block_max(V value) {
+  constexpr int NW = kDtThreads / 32;
+  __shared__ double warps[NW];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll 1
+  for (int w = warp; w < NW; w += blockDim.x >> 5) {
+    const double v = warp_max(value(32 * w + lane));
+    if (lane == 0) warps[w] = v;
+  }
+  __syncthreads();
+  const double v = warp == 0 ? warp_max(lane < NW ? warps[lane] : 0.0) : 0.0;
+  __syncthreads();
+  return v;
+}
+
+// dt of a state with NaNs.  A maximum in the reference's order (a < b ? b : a)
+// keeps a NaN or drops it by the place where it stands, so the cells are folded
+// exactly as the two dt kernels fold them: the first blocks of the grid take
+// dt_partial_kernel's blocks, and the last of them to finish does
+// dt_final_kernel's work.  All threads of those blocks call it; nothing waits for
+// another block.
+template <int D>
+__device__ __noinline__ void redo_dt(const fvh_mesh_view &m, const fvh_state_view &s,
+                                     const next_dt &nd) {
+  __shared__ bool last;
+  const unsigned blocks = min(gridDim.x * gridDim.y, (unsigned)nd.nblocks);
+  for (unsigned b = block_index(); b < (unsigned)nd.nblocks; b += blocks) {
+    const double dt_inv = dt_block_max([&](int i) {
+      double most = 0;
+      for (int c = b * kDtThreads + i; c < m.num_cells; c += nd.nblocks * kDtThreads) {
+        double v[D];
+#pragma unroll
+        for (int j = 0; j < D; ++j) v[j] = s.velocity[j][c];
+        arith_hw hw;
+        most = smax(cell_dt_inv<D, true>(hw, m, c, v, s.sound_speed[c], nd.slot_dx), most);
+      }
+      return most;
+    });
+    if (threadIdx.x == 0) nd.partial[b] = dt_inv;
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicInc(nd.done, blocks - 1) == blocks - 1;  // (back to zero)
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const double dt_inv = dt_block_max([&](int i) {
+    double most = 0;
+    for (int b = i; b < nd.nblocks; b += kDtThreads) most = smax(__ldcg(nd.partial + b), most);
+    return most;
+  });
+  if (threadIdx.x == 0) {
+    *nd.maximum = 0ull;
+    write_dt(dt_inv, nd.cfl, nd.final_time, nd.soln_time, nd.dt, nd.status);
+  }
 }
 __device__ __forceinline__ void add_to_maximum(const next_dt &nd, double dt_inv) {
+  unsigned lo, hi;
+  sf64::halves(dt_inv, lo, hi);
+  if (is_nan(lo, hi)) atomicMax(nd.maximum, kInfinity + 1);
   dt_inv = block_max(dt_inv);
   if (threadIdx.x == 0 && lt(0.0, dt_inv))
     atomicMax(nd.maximum, (unsigned long long)__double_as_longlong(dt_inv));
@@ -1408,17 +1482,19 @@ fluxes_kernel(const __grid_constant__ fvh_mesh_view m, const __grid_constant__ f
   after_previous();
   if (!SECOND) finish_dt(nd);  // (first order has no gradients)
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= m.num_faces) return;
-  const int2 cc = reinterpret_cast<const int2 *>(m.face_cells)[f];
-  double F[D + 2];
-  arith_opt ar;
-  face_flux<D, KIND, SECOND, PRE>(ar, m, s, g, f, cc, swap != 0, outflow != 0, face_dx, F);
-  if (ar.rare) {
-    face_flux_hw<D, KIND, SECOND, PRE>(m, s, g, fl, f, cc, swap, outflow, face_dx);
-    return;
+  if (f < m.num_faces) {
+    const int2 cc = reinterpret_cast<const int2 *>(m.face_cells)[f];
+    double F[D + 2];
+    arith_opt ar;
+    face_flux<D, KIND, SECOND, PRE>(ar, m, s, g, f, cc, swap != 0, outflow != 0, face_dx, F);
+    if (ar.rare) {
+      face_flux_hw<D, KIND, SECOND, PRE>(m, s, g, fl, f, cc, swap, outflow, face_dx);
+    } else {
+      let_next_start();
+      store_flux<D>(fl, f, F);
+    }
   }
-  let_next_start();
-  store_flux<D>(fl, f, F);
+  if (carried_nan(nd)) redo_dt<D>(m, s, nd);
 }
 
 // Few faces (kFewFaces): with the FP64 instructions.
@@ -1429,16 +1505,23 @@ fluxes_few_kernel(const __grid_constant__ fvh_mesh_view m, const __grid_constant
                   const __grid_constant__ fvh_flux_view fl, int swap, int outflow,
                   const double *__restrict__ face_dx, const __grid_constant__ next_dt nd) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= m.num_faces) return;
-  double F[D + 2];
-  arith_hw hw;
-  face_flux<D, KIND, SECOND, PRE>(hw, m, s, g, f, reinterpret_cast<const int2 *>(m.face_cells)[f],
-                                  swap != 0, outflow != 0, face_dx, F, [&] {
-                                    after_previous();
-                                    if (!SECOND) finish_dt(nd);
-                                  });
-  let_next_start();
-  store_flux<D>(fl, f, F);
+  bool nan = false;
+  auto ready = [&] {
+    after_previous();
+    nan = carried_nan(nd);
+    if (!SECOND) finish_dt(nd);
+  };
+  if (f < m.num_faces) {
+    double F[D + 2];
+    arith_hw hw;
+    face_flux<D, KIND, SECOND, PRE>(hw, m, s, g, f, reinterpret_cast<const int2 *>(m.face_cells)[f],
+                                    swap != 0, outflow != 0, face_dx, F, ready);
+    let_next_start();
+    store_flux<D>(fl, f, F);
+  } else {
+    ready();
+  }
+  if (nan) redo_dt<D>(m, s, nd);
 }
 
 // ---------------------------------------------------------------------------

@@ -350,7 +350,9 @@ fvh_status fvh_solver_profile(fvh_solver *s, const fvh_state_view *state,
                               int32_t *launches, int32_t *nkernels,
                               fvh_stream_t stream);
 
-/* Synchronises the stream, reads the status word and the solution time. */
+/* Synchronises the stream, reads the status word and the solution time.  A clear
+ * status word beside a time that is no number (a state with NaNs gave a dt that
+ * is none) is FVH_ERR_INFINITE_DT. */
 fvh_status fvh_solver_check(fvh_solver *s, fvh_stream_t stream,
                             double *soln_time, int64_t *bad_cell);
 

@@ -1566,7 +1566,12 @@ gather_update_kernel(const fvh_mesh_view m, const fvh_state_view s, workspace w,
         }
       }
     };
-    face(0, true);  // (a cell has faces; its first flux is the sum so far)
+    if (nq > 0) {
+      face(0, true);
+    } else {  // (a cell of the caller's without faces)
+#pragma unroll
+      for (int k = 0; k < D + 2; ++k) shi[k] = slo[k] = 0.f;
+    }
     for (int k = 1; k < nq; ++k) face(k, false);
     float vn[D], an;
     cell_update<D, STAGE>(s, w, pk_out, pm, c, pr, sdt.dts, shi, slo, uc, vn, &an,

@@ -865,6 +865,8 @@ __device__ __noinline__ side_limit limiter_side(const fvh_mesh_view &m, const ta
                                                 const double *plane, int c0,
                                                 double u0, double g0, double g1, double g2,
                                                 float E) {
+  const int r0 = m.cell_vertex_offsets[c0], r1 = m.cell_vertex_offsets[c0 + 1];
+  if (r0 == r1) return {okey(1.0), 0u};  // (a cell of the caller's without vertices)
   const double g[3] = {g0, g1, g2};
   unsigned wide = 0, rare = 0;
   float gf[D];
@@ -875,7 +877,6 @@ __device__ __noinline__ side_limit limiter_side(const fvh_mesh_view &m, const ta
 #pragma unroll
     for (int i = 0; i < D; ++i) x0[i] = m.cell_centroid[i][c0];
   }
-  const int r0 = m.cell_vertex_offsets[c0], r1 = m.cell_vertex_offsets[c0 + 1];
   auto estimate = [&](int rr) {
     double dxv[D];
     vertex_offset<D, PRE>(m, t, rr, x0, dxv);

@@ -1,6 +1,7 @@
 """Cells with empty lists, which a caller's own mesh view may hold: one without
-faces, neighbours and vertices (it keeps its state).  They stand last, so that
-nothing follows their place in the lists."""
+faces, neighbours and vertices (it keeps its state), and one without vertices (no
+vertex limits its gradients).  They stand last, so that nothing follows their place
+in the lists."""
 import ctypes as C
 
 import numpy as np
@@ -95,3 +96,37 @@ def test_lone_cell_mixed(cuda, dim, n, schedule):
     assert t == want_t and np.array_equal(out[:, :-1], want)
     # density, velocity and energy stay; the rest is closed from them
     assert np.array_equal(out[:2 + dim, -1], state[:2 + dim, -1])
+
+
+@pytest.mark.parametrize("dim,n", [(2, (24, 17)), (2, (131, 127)), (2, (513, 512)),
+                                   (3, (27, 26, 25)), (3, (46, 45, 46))])
+def test_cell_without_vertices(cuda, oracle_lib, dim, n):
+    """Beside large values the limiter's FP32 bounds do not decide, so it looks for
+    the vertices that do."""
+    a = dict(H.HostMesh.box(dim, n, [0] * dim, [1] * dim, 0.15, 5).arrays())
+    a["cell_vertex_offsets"] = a["cell_vertex_offsets"].copy()
+    a["cell_vertex_offsets"][-1] = a["cell_vertex_offsets"][-2]
+    a["cell_vertices"] = a["cell_vertices"][:a["cell_vertex_offsets"][-1]]
+    mesh = Mesh(cuda, dim, a)
+    nc = mesh.num_cells
+    state = _state(dim, mesh.arrays["cell_centroid"])
+    state[:, -1] += 1.0  # above all neighbours: no room over it
+    state[(0, 1 + dim, 2 + dim, 4 + dim), :] += 1e7
+    p = H.make_params(dim, flux="rusanov", cfl=0.3, final_time=1e9)
+    ds = cuda.tensor(state, device="cuda")
+    dg = cuda.zeros((U.grad_rows(dim), nc), dtype=cuda.float64, device="cuda")
+    sv, gv = U.device_state_view(ds, dim), U.device_gradient_view(dg, dim)
+    cuda.cuda.synchronize()
+    H.check(H.lib().fvh_evaluate_gradients(C.byref(mesh.device.view), C.byref(sv), C.byref(gv),
+                                           C.byref(p), None))
+    cuda.cuda.synchronize()
+    want = U.oracle_gradients(oracle_lib, mesh, state, p)
+    assert np.isfinite(want).all() and np.array_equal(dg.cpu().numpy(), want)
+    dstate = H.DeviceState(dim, nc)
+    solver = H.Solver(mesh.device, p)
+    dstate.upload(state)
+    solver.reset(0.0)
+    solver.step(dstate)
+    out = dstate.download()
+    assert U.oracle_run(oracle_lib, mesh, state, p, 1)[0] == 0
+    assert solver.status()[0] == 0 and np.array_equal(out, state)

@@ -1021,6 +1021,8 @@ constexpr int kStageCells = 128;      // cells per chunk = threads per block
 constexpr int kStageMaxCells = 256;   // staged cell records per chunk (byte slots)
 constexpr int kStageMaxVerts = 256;   // staged vertex records per chunk
 constexpr int kStageMaxBytes = 24576; // one stage buffer at most (two per block)
+// and its list: a head and at most one run a record
+constexpr int kStageMaxListBytes = 16 * (1 + kStageMaxCells + kStageMaxVerts);
 constexpr int kStageWaitPolls = 1 << 22;  // bounded waits on a chunk's copies
 
 template <bool LIMIT>
@@ -1952,7 +1954,7 @@ static cudaError_t setup_stage_host(workspace *w, const fvh_mesh_view &m) {
     }
     units += topo[k].size() / 4;
   }
-  if (t.stage_bytes + 16 * t.list_slots > kStageMaxBytes || units > UINT32_MAX) return cudaSuccess;
+  if (units > UINT32_MAX) return cudaSuccess;
   std::vector<unsigned> blob(4 * units);
   for (int k = 0; k < nchunks; ++k)
     std::copy(topo[k].begin(), topo[k].end(),
@@ -1980,7 +1982,7 @@ static cudaError_t setup_stage_host(workspace *w, const fvh_mesh_view &m) {
   if (e != cudaSuccess) return e;
   // The kernel's limit is the most any mesh may stage, not this mesh's need: it
   // is one setting for all solvers.
-  const int smem = stage_smem(t), most_smem = 2 * kStageMaxBytes;
+  const int smem = stage_smem(t), most_smem = 2 * (kStageMaxBytes + kStageMaxListBytes);
   e = cudaFuncSetAttribute(gradients_staged_kernel<true>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, most_smem);
   if (e == cudaSuccess)

@@ -383,6 +383,7 @@ fvh_status fvh_solver_set_shape(fvh_solver *s, int32_t block, int32_t cells_per_
       (schedule == 2 && fvh::mixed::colours(s->mixed) == 0) ||
       (staged && !fvh::mixed::staging(s->mixed)))
     return FVH_ERR_INVALID_ARGUMENT;
+  if (schedule == 1 && fvh::mixed::bare_cells(s->mixed)) schedule = 0;  // (the same bits)
   s->shape.block = block;
   s->shape.cells_per_thread = cells_per_thread;
   s->shape.schedule = schedule;

@@ -132,6 +132,7 @@ struct workspace {
   stage_tables stage;
   void *stage_base = nullptr;
   int stage_blocks = 0;  // persistent grid
+  bool bare = false;  // some cell has no faces (see bare_cells)
 };
 
 __device__ __forceinline__ void stg256(float4 *p, float4 a, float4 b) {
@@ -1568,12 +1569,7 @@ gather_update_kernel(const fvh_mesh_view m, const fvh_state_view s, workspace w,
         }
       }
     };
-    if (nq > 0) {
-      face(0, true);
-    } else {  // (a cell of the caller's without faces)
-#pragma unroll
-      for (int k = 0; k < D + 2; ++k) shi[k] = slo[k] = 0.f;
-    }
+    face(0, true);  // the first flux is the sum so far (every cell has one: see bare_cells)
     for (int k = 1; k < nq; ++k) face(k, false);
     float vn[D], an;
     cell_update<D, STAGE>(s, w, pk_out, pm, c, pr, sdt.dts, shi, slo, uc, vn, &an,
@@ -1806,6 +1802,8 @@ static cudaError_t setup_colours_host(workspace *w, const fvh_mesh_view &m) {
 
 bool staging(const workspace *w) { return w && w->stage.nchunks > 0; }
 
+bool bare_cells(const workspace *w) { return w && w->bare; }
+
 int colours(const workspace *w) { return w ? w->ncolours : 0; }
 
 // Tables of the staged 2D gradients (see gradients_staged_kernel), built on
@@ -2010,11 +2008,27 @@ static cudaError_t setup_stage(workspace *w, const fvh_mesh_view &m) {
   }
 }
 
+// Whether the caller's mesh has cells without faces (a mesh built by
+// fvh_host_mesh_create has none).
+static cudaError_t setup_bare_cells(workspace *w, const fvh_mesh_view &m) {
+  try {
+    std::vector<int32_t> off(m.num_cells + 1);
+    const cudaError_t e = cudaMemcpy(off.data(), m.cell_face_offsets, sizeof(int32_t) * off.size(),
+                                     cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return e;
+    w->bare = std::adjacent_find(off.begin(), off.end()) != off.end();
+    return cudaSuccess;
+  } catch (const std::bad_alloc &) {
+    return cudaErrorMemoryAllocation;
+  }
+}
+
 fvh_status create(const fvh_mesh_view &m, const fvh_params &p, workspace **out) {
   (void)p;
   const fvh_status r = create_capacity(m.dim, m.num_cells, m.num_faces, m.num_vertices, out);
   if (r != FVH_OK) return r;
   cudaError_t e = setup_geometry(*out, m, nullptr);
+  if (e == cudaSuccess) e = setup_bare_cells(*out, m);
   if (e == cudaSuccess) e = setup_colours(*out, m);
   if (e == cudaSuccess) e = setup_stage(*out, m);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();

@@ -59,6 +59,11 @@ int colours(const workspace *w);
 // Whether the staged gradients serve this workspace's mesh (2D single mesh
 // whose chunks fit the shared-memory stages).
 bool staging(const workspace *w);
+// Whether the mesh has a cell without faces (only a caller's own view can hold
+// one).  The face schedule's gather takes a cell's first flux as its sum so far,
+// so such a mesh runs schedule 0, which gives the same bits, in its place (a test
+// in the gather costs 0.5 % of a 1024^2 step, 0.3 % at 128^3).
+bool bare_cells(const workspace *w);
 
 // Steps of one run on a state nothing else writes in between: the corrector
 // of a step can also write the next step's FP32 pack and dt (the same bits

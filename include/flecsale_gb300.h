@@ -296,7 +296,8 @@ int32_t fvh_solver_launches_per_step(const fvh_solver *s);
  * cell, one flux per face added to its cells' compensated sums; then the
  * update).  Schedules 0 and 1 and all block sizes / cells per thread give the
  * same bits; schedule 2 adds each cell's fluxes in colour order, so its sums
- * round differently (deterministically).  schedule | FVH_SCHEDULE_STAGED (2D
+ * round differently (deterministically).  A mesh with a cell without faces
+ * runs schedule 1 as schedule 0.  schedule | FVH_SCHEDULE_STAGED (2D
  * meshes whose cell chunks fit the stages; FVH_ERR_INVALID_ARGUMENT otherwise)
  * takes the gradients from neighbour records staged in shared memory by the
  * bulk-copy engine, with the same bits.  The FP64 form ignores it.  No

@@ -669,7 +669,9 @@ __global__ void cell_tables_kernel(const fvh_mesh_view m, double *lsq, double *s
       note_odd(dx, odd);
     }
   }
-  for (int q = m.cell_vertex_offsets[c]; q < m.cell_vertex_offsets[c + 1]; ++q) {
+  const int r0 = m.cell_vertex_offsets[c], r1 = m.cell_vertex_offsets[c + 1];
+  if (r0 == r1) atomicOr(odd, 1u);  // a cell without vertices (limiter_side)
+  for (int q = r0; q < r1; ++q) {
     const int v = m.cell_vertices[q];
 #pragma unroll
     for (int d = 0; d < D; ++d) vtx_dx[(size_t)q * D + d] = m.vertex_coord[d][v] - x0[d];
@@ -865,8 +867,6 @@ __device__ __noinline__ side_limit limiter_side(const fvh_mesh_view &m, const ta
                                                 const double *plane, int c0,
                                                 double u0, double g0, double g1, double g2,
                                                 float E) {
-  const int r0 = m.cell_vertex_offsets[c0], r1 = m.cell_vertex_offsets[c0 + 1];
-  if (r0 == r1) return {okey(1.0), 0u};  // (a cell of the caller's without vertices)
   const double g[3] = {g0, g1, g2};
   unsigned wide = 0, rare = 0;
   float gf[D];
@@ -877,6 +877,8 @@ __device__ __noinline__ side_limit limiter_side(const fvh_mesh_view &m, const ta
 #pragma unroll
     for (int i = 0; i < D; ++i) x0[i] = m.cell_centroid[i][c0];
   }
+  const int r0 = m.cell_vertex_offsets[c0], r1 = m.cell_vertex_offsets[c0 + 1];
+  if (!PRE && r0 == r1) return {okey(1.0), 0u};  // (with tables no cell is without vertices)
   auto estimate = [&](int rr) {
     double dxv[D];
     vertex_offset<D, PRE>(m, t, rr, x0, dxv);
@@ -1482,20 +1484,19 @@ fluxes_kernel(const __grid_constant__ fvh_mesh_view m, const __grid_constant__ f
               const __grid_constant__ next_dt nd) {
   after_previous();
   if (!SECOND) finish_dt(nd);  // (first order has no gradients)
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f < m.num_faces) {
-    const int2 cc = reinterpret_cast<const int2 *>(m.face_cells)[f];
-    double F[D + 2];
-    arith_opt ar;
-    face_flux<D, KIND, SECOND, PRE>(ar, m, s, g, f, cc, swap != 0, outflow != 0, face_dx, F);
-    if (ar.rare) {
-      face_flux_hw<D, KIND, SECOND, PRE>(m, s, g, fl, f, cc, swap, outflow, face_dx);
-    } else {
-      let_next_start();
-      store_flux<D>(fl, f, F);
-    }
-  }
   if (carried_nan(nd)) redo_dt<D>(m, s, nd);
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= m.num_faces) return;
+  const int2 cc = reinterpret_cast<const int2 *>(m.face_cells)[f];
+  double F[D + 2];
+  arith_opt ar;
+  face_flux<D, KIND, SECOND, PRE>(ar, m, s, g, f, cc, swap != 0, outflow != 0, face_dx, F);
+  if (ar.rare) {
+    face_flux_hw<D, KIND, SECOND, PRE>(m, s, g, fl, f, cc, swap, outflow, face_dx);
+    return;
+  }
+  let_next_start();
+  store_flux<D>(fl, f, F);
 }
 
 // Few faces (kFewFaces): with the FP64 instructions.
@@ -1798,8 +1799,8 @@ cudaError_t build_tables(const fvh_mesh_view &m, double *base, int64_t nnz_cf,
   t->nbr_dx = nbr_dx;
   t->vtx_dx = vtx_dx;
   t->face_dx = face_dx;
-  // the kernels take these offsets unchecked: a mesh with others computes
-  // them on the fly
+  // the kernels take these offsets unchecked: a mesh with others, or with cells
+  // without vertices, computes them on the fly
   if (odd) t->nbr_dx = t->face_dx = nullptr;
   return cudaSuccess;
 }

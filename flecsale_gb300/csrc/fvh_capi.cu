@@ -371,6 +371,14 @@ static fvh::mixed::step_flags chunk_flags(int64_t k, int64_t n) {
   return f;
 }
 
+// Steps replay graphs of the solver's own, which a stream under capture cannot take:
+// such a call is refused before it touches the graphs or the capture.
+static bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (st == nullptr) return false;
+  return cudaStreamIsCapturing(st, &c) != cudaSuccess || c != cudaStreamCaptureStatusNone;
+}
+
 static fvh_status solver_step_flags(fvh_solver *s, const fvh_state_view *state, cudaStream_t st,
                                     fvh::mixed::step_flags f);
 
@@ -404,6 +412,7 @@ fvh_status fvh_solver_autotune(fvh_solver *s, const fvh_state_view *state, int32
     return FVH_OK;
   }
   cudaStream_t st = cs(stream);
+  if (capturing(st)) return FVH_ERR_CUDA;
   const int D = s->mesh.dim;
   const size_t nc = s->mesh.num_cells;
   // trials run on a scratch copy of the state; the caller's state, solution
@@ -470,7 +479,8 @@ fvh_status fvh_solver_autotune(fvh_solver *s, const fvh_state_view *state, int32
       fvh_solver_set_shape(s, c.block, c.cells_per_thread,
                            c.schedule | (c.staged ? FVH_SCHEDULE_STAGED : 0));
       refresh();
-      // timed as fvh_solver_run launches steps
+      // timed as fvh_solver_run launches steps, but each in a graph of its own (a run
+      // on a small mesh puts several into one)
       fvh_status r = FVH_OK;
       for (int k = 0; k < trial_steps && r == FVH_OK; ++k)
         r = solver_step_flags(s, &tmp, st, chunk_flags(k, trial_steps));
@@ -625,13 +635,6 @@ static bool same_state(fvh_solver *s, const fvh_state_view *state) {
   return false;
 }
 
-// (nothing is built in a stream under capture)
-static bool capturing(cudaStream_t st) {
-  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
-  if (st == nullptr) return false;
-  return cudaStreamIsCapturing(st, &c) != cudaSuccess || c != cudaStreamCaptureStatusNone;
-}
-
 // One step is a fixed sequence of launches; each variant is captured once per
 // state into a CUDA graph and replayed in the caller's stream (the legacy
 // default stream too: the capture runs in a stream of the solver's own).  `steps`
@@ -641,7 +644,6 @@ static fvh_status solver_graph(fvh_solver *s, const fvh_state_view *state, cudaS
   same_state(s, state);
   cudaGraphExec_t &ge = s->graph[steps > 1 ? 4 : (f.pack_first ? 2 : 0) + (f.write_next ? 1 : 0)];
   if (!ge) {
-    if (capturing(st)) return FVH_ERR_CUDA;
     cudaError_t e = cudaSuccess;
     if (!s->capture_stream)
       e = cudaStreamCreateWithFlags(&s->capture_stream, cudaStreamNonBlocking);
@@ -676,7 +678,8 @@ static fvh_status solver_step_flags(fvh_solver *s, const fvh_state_view *state, 
 fvh_status fvh_solver_step(fvh_solver *s, const fvh_state_view *state, fvh_stream_t stream) {
   if (!s || !state_ok(state, s->mesh.dim)) return FVH_ERR_INVALID_ARGUMENT;
   cudaStream_t st = cs(stream);
-  if (!same_state(s, state) && !capturing(st)) return solver_step_enqueue(s, state, st);
+  if (capturing(st)) return FVH_ERR_CUDA;
+  if (!same_state(s, state)) return solver_step_enqueue(s, state, st);
   return solver_step_flags(s, state, st, fvh::mixed::step_flags());
 }
 
@@ -714,14 +717,16 @@ fvh_status fvh_solver_run(fvh_solver *s, const fvh_state_view *state, int64_t ns
                           int32_t stop_at_final_time, int32_t check_every,
                           int64_t *steps_done, fvh_stream_t stream) {
   if (!s || !state_ok(state, s->mesh.dim) || nsteps < 0) return FVH_ERR_INVALID_ARGUMENT;
+  if (steps_done) *steps_done = 0;
+  if (capturing(cs(stream))) return FVH_ERR_CUDA;
   if (check_every <= 0) check_every = 1;
   int64_t n = 0;
   fvh_status r = FVH_OK;
   const double tf = s->params.final_time;
   const double t_stop = tf - 1e-12 * std::fabs(tf);
   const bool apart = s->params.precision == FVH_PRECISION_FP64 && s->mesh.num_cells > kOverlapCells;
-  const bool graphs = same_state(s, state) || capturing(cs(stream)) ||
-                      nsteps >= (apart ? kCaptureStepsApart : kCaptureSteps);
+  const bool graphs =
+      same_state(s, state) || nsteps >= (apart ? kCaptureStepsApart : kCaptureSteps);
   while (n < nsteps) {
     if (stop_at_final_time) {
       double t = 0;

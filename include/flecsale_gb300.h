@@ -264,7 +264,10 @@ fvh_status fvh_solver_create(const fvh_mesh_view *mesh, const fvh_params *params
 void fvh_solver_destroy(fvh_solver *s);
 
 /* One full time step of driver.h:325-375 on the state: dt reduction, then the
- * predictor and the corrector (gradients -> fluxes -> update, factor 0.5 each). */
+ * predictor and the corrector (gradients -> fluxes -> update, factor 0.5 each).
+ * Steps are launched through CUDA graphs of the solver's own, so this call and
+ * fvh_solver_run refuse a stream under capture with FVH_ERR_CUDA (the capture
+ * stays valid); the fvh_evaluate_* / fvh_apply_update tasks can be captured. */
 fvh_status fvh_solver_step(fvh_solver *s, const fvh_state_view *state,
                            fvh_stream_t stream);
 

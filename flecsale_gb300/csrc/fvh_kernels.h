@@ -39,12 +39,11 @@ __device__ __forceinline__ void after_previous() {
 }
 
 template <class... P, class... A>
-inline cudaError_t launch_with(size_t smem, void (*kernel)(P...), dim3 grid, int threads,
-                               cudaStream_t st, bool overlap, const A &...args) {
+inline cudaError_t launch(void (*kernel)(P...), dim3 grid, int threads, cudaStream_t st,
+                          bool overlap, const A &...args) {
   cudaLaunchConfig_t c = {};
   c.gridDim = grid;
   c.blockDim = dim3(threads);
-  c.dynamicSmemBytes = smem;
   c.stream = st;
   cudaLaunchAttribute at = {};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -52,11 +51,6 @@ inline cudaError_t launch_with(size_t smem, void (*kernel)(P...), dim3 grid, int
   c.attrs = &at;
   c.numAttrs = overlap ? 1 : 0;
   return cudaLaunchKernelEx(&c, kernel, P(args)...);
-}
-template <class... P, class... A>
-inline cudaError_t launch(void (*kernel)(P...), dim3 grid, int threads, cudaStream_t st,
-                          bool overlap, const A &...args) {
-  return launch_with(0, kernel, grid, threads, st, overlap, args...);
 }
 
 // Warp-wide maximum with the reference's std::max semantics; all lanes must

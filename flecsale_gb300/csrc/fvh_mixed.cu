@@ -1092,7 +1092,6 @@ gradients_staged_kernel(const fvh_mesh_view m, workspace w, const float4 *__rest
     fetch_list(chunk_of(0), 0);
     if (mine > 1) fetch_list(chunk_of(1), 1);
   }
-  after_previous();
   if (mine > 0) {
     if (tid < 32) {
       landed = __all_sync(0xffffffffu, tma::mbar_wait_bounded(&list_bar[0], 0u, kStageWaitPolls));
@@ -1106,7 +1105,6 @@ gradients_staged_kernel(const fvh_mesh_view m, workspace w, const float4 *__rest
     const unsigned phase = (unsigned)(it >> 1) & 1u;
     const int k = chunk_of(it);
     const int c0 = c_ahead;
-    if (it + 1 == mine) let_next_start();
     // buffers b ^ 1 were last read during the previous chunk (lists: at its
     // start), before the barrier that ended it
     if (it + 1 < mine) {
@@ -2079,11 +2077,11 @@ static void launch_stage_bs(workspace *w, const fvh_mesh_view &m, const fvh_para
     if (D == 2 && staged && w->stage.nchunks > 0 && !pm.cell_problem) {
       const int smem = stage_smem(w->stage);
       if (p.limiter == FVH_LIMITER_NONE)
-        launch_with(smem, gradients_staged_kernel<false>, w->stage_blocks, kStageCells, st, overlap,
-                    m, *w, pk_in, w->stage, dir, pm.status);
+        gradients_staged_kernel<false><<<w->stage_blocks, kStageCells, smem, st>>>(
+            m, *w, pk_in, w->stage, dir, pm.status);
       else
-        launch_with(smem, gradients_staged_kernel<true>, w->stage_blocks, kStageCells, st, overlap, m,
-                    *w, pk_in, w->stage, dir, pm.status);
+        gradients_staged_kernel<true><<<w->stage_blocks, kStageCells, smem, st>>>(
+            m, *w, pk_in, w->stage, dir, pm.status);
     } else if (p.limiter == FVH_LIMITER_NONE) {
       launch(gradients_kernel<D, false, BS>, nb, BS, st, overlap, m, *w, pk_in, dir);
     } else {

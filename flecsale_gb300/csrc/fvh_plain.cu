@@ -712,25 +712,9 @@ __device__ __forceinline__ void load_dx(const double *__restrict__ p, double *dx
   }
 }
 
-// Plane k of the reconstructed variables (d, v.., e, p, a) of a state and of
-// its gradients (component i).
-template <int D>
-__device__ __forceinline__ const double *state_plane(const fvh_state_view &s, int k) {
-  return k == 0 ? s.density
-                : k <= D ? s.velocity[k - 1]
-                         : k == D + 1 ? s.internal_energy
-                                      : k == D + 2 ? s.pressure : s.sound_speed;
-}
-template <int D>
-__device__ __forceinline__ double *grad_plane(const fvh_gradient_view &g, int k, int i) {
-  return k == 0 ? g.density[i]
-                : k <= D ? g.velocity[k - 1][i]
-                         : k == D + 1 ? g.internal_energy[i]
-                                      : k == D + 2 ? g.pressure[i] : g.sound_speed[i];
-}
-
-// ... and the limiter's view of them.  Both views hold their plane pointers one
-// after another, so a variable that is only known at run time is an index.
+// Plane k of the reconstructed variables (d, v.., e, p, a) of a state, and the
+// planes of its gradient.  Both views hold their plane pointers one after another,
+// so a variable that is only known at run time is an index.
 template <int D>
 __device__ __forceinline__ const double *state_plane_at(const fvh_state_view &s, int k) {
   // density, velocity[3], internal_energy, pressure, temperature, sound_speed

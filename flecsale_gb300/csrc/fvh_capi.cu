@@ -59,8 +59,10 @@ struct fvh_solver {
 };
 
 // Launches.  A small mesh's step is a few kernels of 2-10 us, and what lies
-// between them counts: inner steps of a run go kManySteps to a graph (32x32, 20
-// steps: 968 -> 930 us; Sod 100x10 in runs of 10 steps: 2.97 -> 2.79 ms), and up
+// between them counts: inner steps of a run go kManySteps to a graph, which saves
+// about 2 us a step at any size (mixed, us a step, one and four to a graph: 64^2
+// 23.1 and 20.8, 170^2 27.3 and 24.6, 512^2 82.0 and 80.2, 64^3 166.1 and 164.1,
+// 720^2 149.3 and 147.2), so that it no longer counts beyond kManyStepsCells, and up
 // to kOverlapCells cells each FP64 kernel starts while its predecessor ends
 // (930 -> 880 us and 2.67 -> 2.51 ms; 64^2 10 steps 541 -> 511 us; no change at
 // 112^2).  On large meshes a launch is lost in its kernel.

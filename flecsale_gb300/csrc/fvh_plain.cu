@@ -64,8 +64,10 @@ namespace plain {
 // and 68 in pairs, at 112^2 71, 68 and 75; in 3D at 16^3 107, 115 and 132, at
 // 20^3 139, 130 and 152.  Without tables the four tasks take 85 us against 116
 // at 64^2, 111 and 118 at 128^2, 168 and 148 at 200^2.  Fluxes: 11 us a launch against
-// 12.5 with 2,112 faces, both 12.3 with 18,600.  Update: 11 against 11.5 us with
-// 1,024 cells, 19 against 15 with 44,000.
+// 12.5 with 2,112 faces, both 12.3 with 18,600.  Update, a launch in a graph: 4.96
+// us against 5.57 with 1,024 cells, 5.34 and 5.92 with 14,400, 6.56 and 7.02 with
+// 20,022, 6.79 and 7.00 with 28,900, 9.88 and 8.06 with 44,100; in 3D 6.27 against
+// 7.48 with 4,096, 8.60 and 9.15 with 19,683, 10.7 and 9.24 with 32,768.
 constexpr int kFewThreads = 64;
 constexpr int kFewCells = 6144, kFewCellsNoTables = 16384, kFewFaces = 10000;
 constexpr int kFewUpdateCells = 20000;

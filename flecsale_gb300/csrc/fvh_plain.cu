@@ -840,6 +840,16 @@ struct side_limit {
   unsigned rare;
 };
 
+// Whether the sides that FP32 does not decide are taken one by one (limiter_side)
+// or both in limiter_exact.  In 3D without tables each pass gathers the offsets of
+// eight vertices again, and two passes a side cost more than the FP64 sums they
+// save (us, sides and exact: uniform mesh with waves, 28^3 218 and 182, 36^3 272
+// and 239, 54x83x48 851 and 840, 80^3 1,907 and 1,813; jittered 184 and 183, 238
+// and 238, 795 and 836, 1,777 and 1,807; before the FP32 bounds 213, 258, 879 and
+// 1,892).  In 2D the sides win where there are many (800^2 367 and 382).
+template <int D, bool PRE>
+constexpr bool limit_by_sides() { return PRE || D == 2; }
+
 // What one side of the limiter allows a variable whose largest vertex
 // difference above u0 (UP, below u0 otherwise) may exceed the room that the
 // neighbours leave: the order key of min(1, (umax-u0)/du) or of
@@ -958,8 +968,8 @@ __device__ __forceinline__ void solve(A &ar, const double (&r)[10], const double
 // difference du within E of its FP32 estimate, a variable is not limited when
 // du <= tol, or du <= umax - u0 (RN(umax - u0) is the largest neighbour
 // difference, of which the key of the high half gives a lower bound), and
-// likewise below; phi is then 1 exactly.  The other variables take
-// limiter_side.  In flows that are smooth or at rest up to rounding nearly
+// likewise below; phi is then 1 exactly.  The other variables take limiter_side
+// or limiter_exact.  In flows that are smooth or at rest up to rounding nearly
 // all are decided, which saves their vertex products and sums and the second
 // pass over the neighbours.
 template <int D, int NK, bool LIMIT, bool PRE>
@@ -1088,7 +1098,7 @@ __device__ __forceinline__ void cell_gradients(arith_opt &ar, const fvh_mesh_vie
     if (free_up && free_down && !odd) continue;
     long long kphi = okey(1.0);
     const double *gk = gu[k];
-    if (!odd) {
+    if (limit_by_sides<D, PRE>() && !odd) {
       if (!free_up) {
         const side_limit l = limiter_side<D, PRE, true>(m, t, plane[k], c0, u0[k], gk[0], gk[1],
                                                         gk[D - 1], E);
@@ -1103,7 +1113,8 @@ __device__ __forceinline__ void cell_gradients(arith_opt &ar, const fvh_mesh_vie
       }
       kphi = (kphi < 0) ? 0 : kphi;  // std::max(phi, 0)
     }
-    if (odd) kphi = okey(limiter_exact<D, PRE>(m, t, plane[k], c0, u0[k], gk[0], gk[1], gk[D - 1]));
+    if (!limit_by_sides<D, PRE>() || odd)
+      kphi = okey(limiter_exact<D, PRE>(m, t, plane[k], c0, u0[k], gk[0], gk[1], gk[D - 1]));
     if (kphi != okey(1.0)) {
       const auto phi = ar.take(from_okey(kphi));
 #pragma unroll

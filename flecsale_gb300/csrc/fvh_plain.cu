@@ -874,7 +874,6 @@ __device__ __noinline__ side_limit limiter_side(const fvh_mesh_view &m, const ta
     for (int i = 0; i < D; ++i) x0[i] = m.cell_centroid[i][c0];
   }
   const int r0 = m.cell_vertex_offsets[c0], r1 = m.cell_vertex_offsets[c0 + 1];
-  if (!PRE && r0 == r1) return {okey(1.0), 0u};  // (with tables no cell is without vertices)
   auto estimate = [&](int rr) {
     double dxv[D];
     vertex_offset<D, PRE>(m, t, rr, x0, dxv);
@@ -1080,7 +1079,8 @@ __device__ __forceinline__ void cell_gradients(arith_opt &ar, const fvh_mesh_vie
   // E: truncating g and dx and the FP32 roundings move sum |dx g| by less than
   // 2^-21 of itself; values below 2^-60 taken as zero; the reference's own
   // roundings about u0 by less than 2^-50 |u0|.  Each term is taken double.
-  float tiny = 1e-30f;
+  // (A cell without vertices, which a mesh with tables does not have, is free.)
+  float tiny = !PRE && r0 == r1 ? -INFINITY : 1e-30f;
 #pragma unroll
   for (int i = 0; i < D; ++i) tiny = __fmaf_rn(reach[i], 0x1p-59f, tiny);
 #pragma unroll

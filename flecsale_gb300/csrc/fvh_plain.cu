@@ -62,14 +62,21 @@ namespace plain {
 // and unrolled loops load ahead.  Where the lines lie: a step with such gradients
 // takes 58 us at 64^2 against 60 with the integer forms one variable a thread
 // and 68 in pairs, at 112^2 71, 68 and 75; in 3D at 16^3 107, 115 and 132, at
-// 20^3 139, 130 and 152.  Without tables the four tasks take 85 us against 116
-// at 64^2, 111 and 118 at 128^2, 168 and 148 at 200^2.  Fluxes: 11 us a launch against
+// 20^3 139, 130 and 152.  Without tables a gradients launch takes (us, few and many
+// cells' kernel; gas at rest, and waves) in 2D with the limiter 13.3 and 23.0, 14.4
+// and 45.5 at 64^2, 29.4 and 29.3, 29.9 and 46.6 at 112^2, 38.5 and 29.4, 39.8 and
+// 46.4 at 127x129, without it 13.3 and 16.2, 13.3 and 19.9 at 80^2, 19.1 and 16.1,
+// 19.0 and 19.5 at 90^2; in 3D 93 and 107, 92 and 163 at 20^3, 159 and 109, 152 and
+// 162 at 22x23x23, 186 and 111, 187 and 164 at 25x25x26.  Fluxes: 11 us a launch against
 // 12.5 with 2,112 faces, both 12.3 with 18,600.  Update, a launch in a graph: 4.96
 // us against 5.57 with 1,024 cells, 5.34 and 5.92 with 14,400, 6.56 and 7.02 with
 // 20,022, 6.79 and 7.00 with 28,900, 9.88 and 8.06 with 44,100; in 3D 6.27 against
 // 7.48 with 4,096, 8.60 and 9.15 with 19,683, 10.7 and 9.24 with 32,768.
 constexpr int kFewThreads = 64;
-constexpr int kFewCells = 6144, kFewCellsNoTables = 16384, kFewFaces = 10000;
+constexpr int kFewCells = 6144, kFewFaces = 10000;
+constexpr int few_cells_no_tables(int dim, bool limited) {
+  return dim == 3 ? 8000 : limited ? 15360 : 6400;
+}
 constexpr int kFewUpdateCells = 20000;
 
 // Products and quotients in out-of-line calls (a call costs a few
@@ -1737,7 +1744,7 @@ cudaError_t launch_gradients(const fvh_mesh_view &m, const fvh_state_view &s,
                              cudaStream_t st, const tables &t, const next_dt &nd,
                              bool overlap) {
   const bool lim = p.limiter != FVH_LIMITER_NONE, pre = t.lsq && t.nbr_dx && t.vtx_dx;
-  if (m.num_cells <= (pre ? kFewCells : kFewCellsNoTables)) {
+  if (m.num_cells <= (pre ? kFewCells : few_cells_no_tables(D, lim))) {
     const dim3 grid(blocks_of(m.num_cells, kFewThreads), D + 4);
     auto go = [&](auto kernel) { launch(kernel, grid, kFewThreads, st, overlap, m, s, g, t, nd); };
     if (pre)

@@ -59,24 +59,36 @@ namespace plain {
 // Few cells or faces leave most of the chip idle and a kernel's time is one
 // thread's chain of loads and operations.  The FP64 instructions are then the
 // shorter chain (their pipe is shared by few warps), small blocks reach more SMs
-// and unrolled loops load ahead.  Where the lines lie: a step with such gradients
-// takes 58 us at 64^2 against 60 with the integer forms one variable a thread
-// and 68 in pairs, at 112^2 71, 68 and 75; in 3D at 16^3 107, 115 and 132, at
-// 20^3 139, 130 and 152.  Without tables a gradients launch takes (us, few and many
-// cells' kernel; gas at rest, and waves) in 2D with the limiter 13.3 and 23.0, 14.4
-// and 45.5 at 64^2, 29.4 and 29.3, 29.9 and 46.6 at 112^2, 38.5 and 29.4, 39.8 and
-// 46.4 at 127x129, without it 13.3 and 16.2, 13.3 and 19.9 at 80^2, 19.1 and 16.1,
-// 19.0 and 19.5 at 90^2; in 3D 93 and 107, 92 and 163 at 20^3, 159 and 109, 152 and
-// 162 at 22x23x23, 186 and 111, 187 and 164 at 25x25x26.  Fluxes: 11 us a launch against
-// 12.5 with 2,112 faces, both 12.3 with 18,600.  Update, a launch in a graph: 4.96
-// us against 5.57 with 1,024 cells, 5.34 and 5.92 with 14,400, 6.56 and 7.02 with
-// 20,022, 6.79 and 7.00 with 28,900, 9.88 and 8.06 with 44,100; in 3D 6.27 against
-// 7.48 with 4,096, 8.60 and 9.15 with 19,683, 10.7 and 9.24 with 32,768.
+// and unrolled loops load ahead.  Where the lines lie:
 constexpr int kFewThreads = 64;
-constexpr int kFewCells = 6144, kFewFaces = 10000;
+// Gradients with tables: a step takes 58 us at 64^2 against 60 with the integer forms
+// one variable a thread and 68 in pairs, at 112^2 71, 68 and 75; in 3D at 16^3 107,
+// 115 and 132, at 20^3 139, 130 and 152.
+constexpr int kFewCells = 6144;
+// ... and without (us a launch, few and many cells' kernel; gas at rest, and waves):
+// 2D with the limiter 13.3 and 23.0, 14.4 and 45.5 at 64^2, 29.4 and 29.3, 29.9 and
+// 46.6 at 112^2, 38.5 and 29.4, 39.8 and 46.4 at 127x129; without it 13.3 and 16.2,
+// 13.3 and 19.9 at 80^2, 19.1 and 16.1, 19.0 and 19.5 at 90^2; 3D 93 and 107, 92 and
+// 163 at 20^3, 159 and 109, 152 and 162 at 22x23x23, 186 and 111, 187 and 164 at
+// 25x25x26.
 constexpr int few_cells_no_tables(int dim, bool limited) {
   return dim == 3 ? 8000 : limited ? 15360 : 6400;
 }
+// Fluxes: a step with tables takes 44.0 us against 48.1 (HLLE), 45.1 and 45.7 (HLLC),
+// 43.2 and 44.7 (Rusanov) at 64^2, 58.1 and 59.7, 59.4 and 57.4, 56.1 and 56.0 at
+// 100^2; in 3D 71.5 and 74.7, 71.6 and 72.8, 70.9 and 71.8 at 12^3.  First order 5.8
+// us a launch against 6.8, 6.1 and 6.2, 5.1 and 5.8 at 64^2.  Second order without
+// tables only Rusanov gains (7.1 and 7.7, in 3D 10.1 and 10.5): HLLC takes 8.7 and
+// 7.0 on a gas at rest and 8.2 and 8.4 with waves at 64^2, 11.7 and 8.2, 11.1 and
+// 10.9 at 12^3, HLLE 7.8 and 7.8, 11.0 and 9.4.
+constexpr int kFewFaces = 10000;
+constexpr bool few_faces_form(int kind, bool second, bool pre) {
+  return pre || !second || kind == FVH_FLUX_RUSANOV;
+}
+// Update, a launch in a graph: 4.96 us against 5.57 with 1,024 cells, 5.34 and 5.92
+// with 14,400, 6.56 and 7.02 with 20,022, 6.79 and 7.00 with 28,900, 9.88 and 8.06
+// with 44,100; in 3D 6.27 against 7.48 with 4,096, 8.60 and 9.15 with 19,683, 10.7 and
+// 9.24 with 32,768.
 constexpr int kFewUpdateCells = 20000;
 
 // Products and quotients in out-of-line calls (a call costs a few
@@ -1820,10 +1832,13 @@ static void launch_fluxes_kind(const fvh_mesh_view &m, const fvh_state_view &s,
   };
   auto kind = [&](auto k) {
     constexpr int KIND = decltype(k)::value;
-    if (m.num_faces <= kFewFaces)
-      go(fluxes_few_kernel<D, KIND, SECOND, PRE>, kFewThreads);
-    else
-      go(fluxes_kernel<D, KIND, SECOND, PRE>, kFaceThreads);
+    if constexpr (few_faces_form(KIND, SECOND, PRE)) {
+      if (m.num_faces <= kFewFaces) {
+        go(fluxes_few_kernel<D, KIND, SECOND, PRE>, kFewThreads);
+        return;
+      }
+    }
+    go(fluxes_kernel<D, KIND, SECOND, PRE>, kFaceThreads);
   };
   if (p.flux_kind == FVH_FLUX_RUSANOV)
     kind(std::integral_constant<int, FVH_FLUX_RUSANOV>());

@@ -34,3 +34,24 @@ def test_gradients(cuda, oracle_lib, dim, n, limiter, jitter):
                                            C.byref(p), None))
     cuda.cuda.synchronize()
     assert np.array_equal(dg.cpu().numpy(), U.oracle_gradients(oracle_lib, mesh, state, p))
+
+
+# 9,940 faces and 10,081; 6,072 and 10,095
+@pytest.mark.parametrize("dim,n", [(2, (70, 70)), (2, (71, 70)), (3, (12, 12, 13)), (3, (15, 15, 14))])
+@pytest.mark.parametrize("flux", ["hlle", "hllc", "rusanov"])
+@pytest.mark.parametrize("order", [1, 2])
+def test_fluxes(cuda, oracle_lib, dim, n, flux, order):
+    mesh = H.HostMesh.box(dim, n, [0] * dim, [1] * dim, 0.15, 5)
+    p = H.make_params(dim, flux=flux, order=order, cfl=0.3)
+    state = _state(dim, mesh.arrays()["cell_centroid"])
+    grads = U.oracle_gradients(oracle_lib, mesh, state, p)
+    dmesh = H.DeviceMesh(mesh)
+    ds, dg = (cuda.tensor(a, device="cuda") for a in (state, grads))
+    df = cuda.zeros((dim + 2, mesh.num_faces), dtype=cuda.float64, device="cuda")
+    sv, gv = U.device_state_view(ds, dim), U.device_gradient_view(dg, dim)
+    fv = U.device_flux_view(df, dim)
+    cuda.cuda.synchronize()
+    H.check(H.lib().fvh_evaluate_fluxes(C.byref(dmesh.view), C.byref(sv), C.byref(gv), C.byref(fv),
+                                        C.byref(p), None))
+    cuda.cuda.synchronize()
+    assert np.array_equal(df.cpu().numpy(), U.oracle_fluxes(oracle_lib, mesh, state, grads, p))
